@@ -11,7 +11,7 @@ binned paths trade a counting sort for cache-friendly gathers.
 
 The tuner times each candidate with CUDA events on the caller's own query
 rows (evaluating a scratch copy, so the caller's array is untouched),
-caches the winner in memory and in a JSON file keyed by GPU, dimension,
+caches the winner in memory and in a JSON file keyed by GPU, kernels, dimension,
 field count, precision and the log2 buckets of cell and query counts, and
 reuses it for every later batch of that shape.  Set ARBINTERP_TUNE_DIR to
 move the cache file, or ARBINTERP_TUNE=off to use the built-in defaults.
@@ -29,6 +29,7 @@ from . import _lib
 
 _MEM: dict = {}
 _LOCK = threading.Lock()
+KERNELS = 2                     # generation of the query kernels: plans measured on another are not reused
 TABLE_TUNE_BYTES = 4 << 30      # only try the table strategy when it is this small or already built
 
 
@@ -73,7 +74,7 @@ def plan_key(interp, nq):
     if dev is None:
         dev = _NAMES[interp.device] = torch.cuda.get_device_name(interp.device)
     b = lambda v: int(math.log2(max(v, 1)))  # noqa: E731
-    return (f"{dev}|d{interp._dim}|F{interp._F}|{interp.precision}|cells2^{b(interp.nc)}|"
+    return (f"{dev}|k{KERNELS}|d{interp._dim}|F{interp._F}|{interp.precision}|cells2^{b(interp.nc)}|"
             f"q2^{b(nq)}|table{int(interp._table_complete)}")
 
 

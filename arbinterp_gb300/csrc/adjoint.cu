@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(256) adjoint3_kernel(arb_grid g, KParams kp, c
   if constexpr (MIXED)
     s = coord_step_fast<3>(qv, kp.ax, g, fr);
   else
-    s = coord_step<3, true>(qv, g, kp.inv_h, fr);
+    s = coord_step_fx<3>(qv, kp.ax, g, fr);
   const bool dead = s.oob || s.nan || s.idx >= g.nc;
   if (!s.oob && !s.nan && s.idx > g.nc) set_status(status, ARB_ERR_CELL_INDEX);
   if (dead) {

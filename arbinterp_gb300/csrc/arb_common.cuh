@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <type_traits>
 
@@ -97,51 +98,6 @@ struct CoordStep {
   bool nan;          // some coordinate NaN (row not rewritten, outputs NaN)
 };
 
-// exact == true: IEEE division (used by the float64 path).
-// exact == false: multiply by 1/h and fall back to the division only when the
-// product lies within a few ulps of an integer, so floor() still matches.
-template <int DIM, bool EXACT>
-__device__ __forceinline__ CoordStep coord_step(const double *qrow, const arb_grid &g,
-                                                const double *inv_h, double frac[DIM]) {
-  CoordStep s;
-  s.oob = false;
-  s.nan = false;
-  int64_t fl[DIM];
-#pragma unroll
-  for (int a = 0; a < DIM; ++a) {
-    const double q = qrow[a];
-    if (q < g.lo[a] || q > g.hi[a]) s.oob = true;
-    if (q != q) s.nan = true;
-    const double d = q - g.lo[a];
-    double iu, k;
-    if (EXACT) {
-      iu = d / g.h[a];
-      k = floor(iu);
-    } else {
-      iu = d * inv_h[a];
-      k = floor(iu);
-      const double guard = fmax(fabs(iu), 1.0) * 1.7763568394002505e-15;  // 8 ulp(1)
-      if (iu - k < guard || (k + 1.0) - iu < guard) {
-        iu = d / g.h[a];
-        k = floor(iu);
-      }
-    }
-    frac[a] = iu - k;
-    fl[a] = (int64_t)k;
-  }
-#pragma unroll
-  for (int a = 0; a < DIM; ++a) s.fl[a] = fl[a];
-  if (s.oob || s.nan) {
-    s.idx = g.nc;
-    return s;
-  }
-  int64_t idx = fl[DIM - 1];
-#pragma unroll
-  for (int a = DIM - 2; a >= 0; --a) idx = idx * (g.n[a] - 3) + fl[a];
-  s.idx = idx;
-  return s;
-}
-
 // Order-preserving map of a double onto uint64: a < b <=> key(a) < key(b)
 // for non-NaN values, so bounds tests run on the integer pipe.
 __host__ __device__ __forceinline__ unsigned long long ord_key_bits(unsigned long long b) {
@@ -163,7 +119,41 @@ struct FastAxis {
   double lo, h, inv_h;
   float loh, lol, ih, il;             // float32 pairs of IntMin and 1/h
   int df;                             // the float32 double-float step applies on this axis
+  unsigned long long hm, hinv;        // significand of h (53 bits) and floor(2^115 / hm), for axis_step_fx
+  int he;                             // biased exponent of h; 0 where axis_step_fx does not apply
 };
+
+// Constants of axis_step_fx: h normal, finite and positive.  floor(2^115 / hm)
+// by a float64 quotient (53 of its 63 bits) and two integer corrections.
+__host__ __device__ inline void fast_axis_fx(FastAxis &f, double h) {
+#ifdef __CUDA_ARCH__
+  const unsigned long long b = (unsigned long long)__double_as_longlong(h);
+#else
+  unsigned long long b;
+  memcpy(&b, &h, 8);
+#endif
+  const int e = (int)(b >> 52);  // with the sign: a negative h is out of range
+  f.he = 0;
+  f.hm = f.hinv = 1ULL << 62;
+  if (e < 64 || e > 1983) return;
+  f.he = e;
+  f.hm = (b & 0xfffffffffffffULL) | 0x10000000000000ULL;
+  unsigned long long q = (unsigned long long)(0x1p115 / (double)f.hm);  // in (2^62, 2^63]
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k) {
+    const __int128 r = ((__int128)1 << 115) - (__int128)q * (__int128)f.hm;
+    q += (long long)((double)(long long)(r >> 20) / ((double)f.hm * 0x1p-20));
+  }
+#pragma unroll 1
+  for (int k = 0; k < 4; ++k) {  // exact: 0 <= 2^115 - q hm < hm
+    const __int128 r = ((__int128)1 << 115) - (__int128)q * (__int128)f.hm;
+    if (r < 0)
+      --q;
+    else if (r >= (__int128)f.hm)
+      ++q;
+  }
+  f.hinv = q;
+}
 
 // Float32 pairs of IntMin and 1/h, and whether the double-float step of
 // coord_step_fast applies: the interpolation range spans at most 2^20 cells
@@ -239,6 +229,117 @@ static __device__ __noinline__ AxisStep axis_step_f64(double q, const FastAxis &
   r.k = kk;
   r.fr = fr;
   return r;
+}
+
+// ---- coordinate step in float64, on the integer pipe --------------------------
+// iu = (q - IntMin) / h with IEEE rounding, its floor and iu - floor(iu), bit
+// for bit as float64 arithmetic gives them.  The division, compares, floor and
+// conversions would be ~17 float64-pipe operations per axis at 2 lanes per SM
+// and clock (binning passes of 1e7 rows: 0.72 + 1.02 ms); here all but the
+// subtraction are integer operations (0.16 + 0.57 ms).
+// fx_quotient: the significand quotient md / hm by the reciprocal hinv; the
+// estimate is low by at most one, the remainder (exact modulo 2^64) corrects
+// and rounds it.  A quotient of two 53-bit significands is never halfway
+// between two 53-bit values.
+__host__ __device__ __forceinline__ unsigned long long fx_mulhi(unsigned long long a, unsigned long long b) {
+#ifdef __CUDA_ARCH__
+  return __umul64hi(a, b);
+#else
+  return (unsigned long long)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
+// Floor (returned) and fraction (float64 bits) of the float64 quotient of
+// the positive normal d (bits) by the axis' h; false where the fixed-point
+// step does not apply (the caller divides).
+__host__ __device__ __forceinline__ bool fx_quotient(unsigned long long d, unsigned long long hm,
+                                                     unsigned long long hinv, int he, long long &k,
+                                                     unsigned long long &frac) {
+  const int ed = (int)(d >> 52);
+  const unsigned long long md = (d & 0xfffffffffffffULL) | 0x10000000000000ULL;
+  const bool ge = md >= hm;
+  unsigned long long Q = fx_mulhi(md << 11, hinv) >> (ge ? 10 : 9);
+  unsigned long long rem = (md << (ge ? 52 : 53)) - Q * hm;
+  if (rem >= hm) {
+    ++Q;
+    rem -= hm;
+  }
+  if (rem + rem > hm) ++Q;
+  int nf = 52 - (ed - he - (ge ? 0 : 1));  // iu = Q 2^-nf
+  if (Q >> 53) {
+    Q >>= 1;
+    --nf;
+  }
+  // quotients from 2^31 (and d = 0 or subnormal, which have no implicit one) are the caller's
+  if (ed == 0 || ed > 2046 || he == 0 || nf < 22 || nf > 900) return false;
+  unsigned long long f = Q;
+  k = 0;
+  if (nf < 64) {
+    k = (long long)(Q >> nf);
+    f = Q & ((1ULL << nf) - 1ULL);
+  }
+  if (f == 0) {
+    frac = 0;
+    return true;
+  }
+#ifdef __CUDA_ARCH__
+  const int z = __clzll((long long)f);
+#else
+  const int z = __builtin_clzll(f);
+#endif
+  frac = ((unsigned long long)(1023 + 62 - z - nf) << 52) + (f << (z - 11));
+  return true;
+}
+
+struct AxisStep64 {
+  double iu, k;
+};
+static __device__ __noinline__ AxisStep64 axis_step_div(double d, double h) {
+  AxisStep64 r;
+  r.iu = d / h;
+  r.k = floor(r.iu);
+  return r;
+}
+
+template <int DIM>
+__device__ __forceinline__ CoordStep coord_step_fx(const double *qrow, const FastAxis *ax, const arb_grid &g,
+                                                   double frac[DIM]) {
+  CoordStep s;
+  s.oob = false;
+  s.nan = false;
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) {
+    const double q = qrow[a];
+    const unsigned long long qb = opaque_u64((unsigned long long)__double_as_longlong(q));
+    const bool isnan = (qb & 0x7fffffffffffffffULL) > 0x7ff0000000000000ULL;
+    const unsigned long long key = ord_key_bits(qb);
+    const bool out = !isnan && (key < ax[a].lo_key || key > ax[a].hi_key);
+    s.nan |= isnan;
+    s.oob |= out;
+    s.fl[a] = 0;
+    frac[a] = 0.0;
+    if (isnan || out) continue;
+    const double d = __dsub_rn(q, ax[a].lo);
+    long long k;
+    unsigned long long fb;
+    if (fx_quotient(opaque_u64((unsigned long long)__double_as_longlong(d)), ax[a].hm, ax[a].hinv, ax[a].he, k, fb)) {
+      s.fl[a] = k;
+      frac[a] = __longlong_as_double((long long)fb);
+    } else if (__double_as_longlong(d) != 0) {
+      const AxisStep64 r = axis_step_div(d, ax[a].h);
+      s.fl[a] = (int64_t)r.k;
+      frac[a] = r.iu - r.k;
+    }
+  }
+  if (s.oob || s.nan) {
+    s.idx = g.nc;
+    return s;
+  }
+  int64_t idx = s.fl[DIM - 1];
+#pragma unroll
+  for (int a = DIM - 2; a >= 0; --a) idx = idx * (g.n[a] - 3) + s.fl[a];
+  s.idx = idx;
+  return s;
 }
 
 template <int DIM>

@@ -28,6 +28,7 @@ __device__ void make_kparams_axis(const arb_grid &g, int a, KParams &kp) {
   kp.ax[a].h = h;
   kp.ax[a].inv_h = 1.0 / h;
   fast_axis_pairs(kp.ax[a], lo, hi, h);
+  fast_axis_fx(kp.ax[a], h);
 }
 
 // One warp takes the next tile from the counter and fills descriptor slot
@@ -100,7 +101,7 @@ __device__ __forceinline__ void batched_rows(const arb_grid &g, const KParams &k
 // the take (counter, field search, descriptor) do not hold the CTA at the
 // barrier between tiles.
 template <bool MIXED, int FF>
-__global__ void __launch_bounds__(256, MIXED ? 2 : 1) batched_kernel(const arb_grid *grids, int32_t nfields,
+__global__ void __launch_bounds__(256, 2) batched_kernel(const arb_grid *grids, int32_t nfields,
                                                       const int64_t *q_off, const int64_t *tile_off,
                                                       int64_t ntiles, int32_t tile_rows, double *q,
                                                       int64_t qs, int wb, arb_query_out o,

@@ -11,16 +11,17 @@
 //   * table (tab_*): gathers the cell's coefficient row(s) and evaluates the
 //     monomial sum by Horner's rule.
 //
-// Precision: FP64 evaluates in float64 with IEEE division for the cell
-// index.  MIXED reads the (hi, lo) float32 split of the grid (or a float32
-// table) and evaluates in float32; the cell index and fractional offset are
-// still formed in float64 so indices and NaN masks are bit-exact.
+// Precision: FP64 forms cell index and fraction as the IEEE quotient gives
+// them and contracts the float64 grid in block fixed point (fx.cuh; the table
+// in float64 arithmetic).  MIXED reads the (hi, lo) float32 split of the grid
+// (or a float32 table) and evaluates in float32; the cell index is that of the
+// float64 step, so indices and NaN masks are bit-exact.
 #include "eval.cuh"
 
 namespace arb {
 
 template <int F, bool MIXED>
-__global__ void __launch_bounds__(256) otf3_kernel(arb_grid g, KParams kp, double *q, int64_t nq,
+__global__ void __launch_bounds__(256, MIXED ? 1 : 2) otf3_kernel(arb_grid g, KParams kp, double *q, int64_t nq,
                                                    int64_t qs, int wb, arb_query_out o,
                                                    int32_t *status) {
   using T = typename std::conditional<MIXED, float, double>::type;
@@ -38,7 +39,7 @@ __global__ void __launch_bounds__(256) otf3_kernel(arb_grid g, KParams kp, doubl
 }
 
 template <int F, bool MIXED>
-__global__ void __launch_bounds__(128) otf4_kernel(arb_grid g, KParams kp, double *q, int64_t nq,
+__global__ void __launch_bounds__(128, MIXED ? 1 : 3) otf4_kernel(arb_grid g, KParams kp, double *q, int64_t nq,
                                                    int64_t qs, int wb, arb_query_out o,
                                                    int32_t *status) {
   using T = typename std::conditional<MIXED, float, double>::type;

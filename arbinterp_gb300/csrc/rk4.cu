@@ -26,7 +26,7 @@ __device__ __forceinline__ bool rk4_accel(const arb_grid &g, const KParams &kp, 
   if constexpr (MIXED)
     s = coord_step_fast<3>(x, kp.ax, g, fr);
   else
-    s = coord_step<3, true>(x, g, kp.inv_h, fr);
+    s = coord_step_fx<3>(x, kp.ax, g, fr);
   if (s.oob || s.nan || s.idx >= g.nc) return false;
   int64_t c[3];
   cell_from_step<3>(s, g, c);
@@ -38,7 +38,7 @@ __device__ __forceinline__ bool rk4_accel(const arb_grid &g, const KParams &kp, 
 }
 
 template <int F, bool MIXED>
-__global__ void __launch_bounds__(128) rk4_kernel(arb_grid g, KParams kp, double *state, int64_t n, double dt,
+__global__ void __launch_bounds__(128, MIXED ? 1 : 3) rk4_kernel(arb_grid g, KParams kp, double *state, int64_t n, double dt,
                                                   int64_t nsteps, double coef, double g0, double g1, double g2,
                                                   double *path, int64_t rec_every, unsigned long long *lost) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

@@ -78,8 +78,8 @@ struct BinGeom {
   int64_t nb[4];     // bins per axis
   int64_t nbins;     // product
   int shift;         // log2 cells per bin edge
-  int cls;           // log2 bank classes per bin (4: 3D mixed 8^3-cell bins and 4D mixed scalar
-                     // 4^4-cell bins; 0 otherwise)
+  int cls;           // log2 bank classes per bin (4: 3D 8^3-cell bins and 4D 4^4-cell bins, in mixed
+                     // precision of scalar fields only; 0 otherwise)
   int64_t nsub;      // nbins << cls sub-bins (bin-major); the special sub-bin is index nsub
 };
 
@@ -117,10 +117,8 @@ static inline BinGeom bin_geom(const arb_grid *g, int precision) {
     b.nbins *= b.nb[a];
   }
   b.cls = 0;
-  if (precision == ARB_PREC_MIXED) {
-    if (g->dim == 3 && b.shift == 3) b.cls = 4;
-    if (g->dim == 4 && b.shift == 2 && g->nfield == 1) b.cls = 4;
-  }
+  if (g->dim == 3 && b.shift == 3) b.cls = 4;
+  if (g->dim == 4 && b.shift == 2 && (g->nfield == 1 || precision != ARB_PREC_MIXED)) b.cls = 4;
   b.nsub = b.nbins << b.cls;
   return b;
 }
@@ -165,7 +163,7 @@ __device__ __forceinline__ CoordStep bin_step(const arb_grid &g, const KParams &
   for (int a = 0; a < DIM; ++a) qv[a] = qr[a];
   CoordStep s;
   if constexpr (EXACT)
-    s = coord_step<DIM, true>(qv, g, kp.inv_h, frac);
+    s = coord_step_fx<DIM>(qv, kp.ax, g, frac);
   else
     s = coord_step_fast<DIM>(qv, kp.ax, g, frac);
   bin = bg.nsub;
@@ -390,7 +388,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const uint32_t
 }
 
 template <int DIM, int F, bool MIXED, bool TABLE>
-__global__ void __launch_bounds__(DIM == 3 ? 256 : 128) eval_sorted_kernel(arb_grid g, KParams kp,
+__global__ void __launch_bounds__(DIM == 3 ? 256 : 128, MIXED ? 1 : (DIM == 3 ? 2 : 3)) eval_sorted_kernel(arb_grid g, KParams kp,
                                                                            int64_t nq, arb_query_out o,
                                                                            SortedWork w) {
   using T = typename std::conditional<MIXED, float, double>::type;
@@ -798,6 +796,10 @@ static bool launch_eval_bin4(const arb_grid *g, const KParams &kp, const BinGeom
   return true;
 }
 
+}  // namespace arb
+#include "fx_tile.cuh"
+namespace arb {
+
 template <int DIM, bool MIXED>
 static void launch_bin(const arb_grid *g, const KParams &kp, const BinGeom &bg, double *q, int64_t nq,
                        int64_t qs, int wb, const arb_query_out *out, int32_t *status, const SortedWork &w,
@@ -923,6 +925,7 @@ static void launch_eval(const arb_grid *g, const KParams &kp, int64_t nq, const 
   const BinGeom bg = bin_geom(g, MIXED ? ARB_PREC_MIXED : ARB_PREC_FP64);
   if (DIM == 3 && MIXED && !table && launch_eval_binc(g, kp, bg, nq, out, w, s)) return;
   if (DIM == 4 && MIXED && !table && launch_eval_bin4(g, kp, bg, nq, out, w, s)) return;
+  if (!MIXED && !table && launch_eval_fx<DIM>(g, kp, bg, nq, out, w, s)) return;
   const int TE = DIM == 3 ? 256 : 128;
   const unsigned BE = (unsigned)((nq + TE - 1) / TE);
 #define ES(FF, TAB) eval_sorted_kernel<DIM, FF, MIXED, TAB><<<BE, TE, 0, s>>>(*g, kp, nq, *out, w)
