@@ -238,6 +238,9 @@ __host__ __device__ __forceinline__ void fx_eval3(const SRC &src, const FxW &wx,
 // integers, kept 2^-5 down so that T_c fits (the correction's weights are at
 // most 0.074^4, its derivatives' 0.5 0.074^3).  Derivative weights are stored
 // times 2^-2 (DS = 2).  GRADF: also the derivatives (times 2^-2) into G.
+// SRC::UNROLL: planes of a slab unrolled (words from a tile) or in a loop (with
+// the conversions of a gathered block the body would outgrow the instruction
+// cache).
 template <bool GRADF, class SRC>
 __host__ __device__ __forceinline__ void fx_eval4(const SRC &src, const FxW w[4], long long &R, long long G[4]) {
   FxAcc<3> V, gt;
@@ -252,13 +255,15 @@ __host__ __device__ __forceinline__ void fx_eval4(const SRC &src, const FxW w[4]
     long long E2[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) E2[m] = 0;
-#pragma unroll 1
+#pragma unroll SRC::UNROLL
     for (int k = 0; k < 4; ++k) {
       FxAcc<2> Y, yx;
       FxAcc<3> yy;
-      long long E1[4];  // slots (x corner) + 2 (y corner) of the x, y differences, times 2^-5
       FxAcc<1> a[4];
       FxAcc<2> d[4];
+      // words of the x, y differences of corner (m & 1, m >> 1): sums of four
+      // samples, the low words 2^-3 down so that they fit
+      int eh[4], el[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -267,11 +272,10 @@ __host__ __device__ __forceinline__ void fx_eval4(const SRC &src, const FxW w[4]
           src.point(i, j, k, t, &h, &l);
           a[j].mac(h, l, w[0].wh[i], w[0].wl[i]);
           if (GRADF) d[j].mac(h, l, w[0].dh[i], w[0].dl[i]);
-          // + at (i, j) both in the upper or both in the lower half of the difference
-          const int sg = ((i >= 2) == (j >= 2)) ? 1 << 27 : -(1 << 27);
           const int m = (i & 1) + 2 * (j & 1);
-          const long long low = ((i >= 2) == (j >= 2)) ? (l >> 5) : -(l >> 5);
-          E1[m] = fx_mad(h, sg, i < 2 && j < 2 ? low : E1[m] + low);
+          const bool plus = (i >= 2) == (j >= 2);  // both in the upper or both in the lower half of the difference
+          eh[m] = i < 2 && j < 2 ? h : (plus ? eh[m] + h : eh[m] - h);
+          el[m] = i < 2 && j < 2 ? l >> 3 : (plus ? el[m] + (l >> 3) : el[m] - (l >> 3));
         }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -295,12 +299,13 @@ __host__ __device__ __forceinline__ void fx_eval4(const SRC &src, const FxW w[4]
         yy.norm(h, l);
         zy.mac(h, l, wh, wl);
       }
-      const long long sg = k >= 2 ? 0 : -1;
+      const long long up = k >= 2 ? 0 : -1, even = (k & 1) - 1;
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const long long v = (E1[m] ^ sg) - sg;
-        E2[m] += (k & 1) ? 0 : v;
-        E2[m + 4] += (k & 1) ? v : 0;
+      for (int m = 0; m < 4; ++m) {  // times 2^-5
+        const long long e = (long long)((unsigned long long)(long long)eh[m] << 27) + (el[m] >> 2);
+        const long long v = (e ^ up) - up;
+        E2[m] += v & even;
+        E2[m + 4] += v & ~even;
       }
     }
     const int wh = fx_sel(w[3].wh, t), wl = fx_sel(w[3].wl, t);
@@ -316,12 +321,12 @@ __host__ __device__ __forceinline__ void fx_eval4(const SRC &src, const FxW w[4]
       zz.norm(h, l);
       gz.mac(h, l, wh, wl);
     }
-    const long long sg = t >= 2 ? 0 : -1;
+    const long long up = t >= 2 ? 0 : -1, even = (t & 1) - 1;
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
-      const long long v = (E2[m] ^ sg) - sg;
-      S[m] += (t & 1) ? 0 : v;
-      S[m + 8] += (t & 1) ? v : 0;
+      const long long v = (E2[m] ^ up) - up;
+      S[m] += v & even;
+      S[m + 8] += v & ~even;
     }
   }
   // correction: contract T_c (units 2^5) with (-w0, w3) along x, y, z, t; with
@@ -434,10 +439,11 @@ struct FxMax {
     m = max(m, hi & 0x7fffffffu);
     z |= lo;
   }
-  // Exponent for the scaling; false where it does not apply (infinities,
-  // NaN, magnitudes outside 2^[-959, 1017]).  All zeros: any exponent.
+  // Exponent for the scaling, one more for a sample that rounds up to the next
+  // (then four high words add up in 32 bits); false where it does not apply
+  // (infinities, NaN, magnitudes outside 2^[-959, 1017]).  All zeros: any.
   __device__ __forceinline__ bool exponent(int &e) const {
-    e = (int)(m >> 20);
+    e = (int)((m + 1) >> 20);
     if ((m | z) == 0) e = 1023;
     return e >= FX_EMIN && e <= FX_EMAX;
   }
@@ -470,7 +476,7 @@ struct FxGrid3 {
   __device__ __forceinline__ bool fit() const {
     bool ok = true;
 #pragma unroll
-    for (int f = 0; f < F; ++f) ok &= (int)(over[f] >> 20) <= emax[f];
+    for (int f = 0; f < F; ++f) ok &= (int)((over[f] + 1) >> 20) <= emax[f];
     return ok;
   }
   // FULL: the whole block, exactly; otherwise the cell's corners, with headroom
@@ -505,6 +511,7 @@ struct FxGrid3 {
 
 // One field of a 4D block; points lie `step` doubles apart along x.
 struct FxGrid4 {
+  static constexpr int UNROLL = 1;
   const double *p;
   int64_t step, sy, sz, st;
   int emax;
@@ -518,7 +525,7 @@ struct FxGrid4 {
     over = max(over, hi & 0x7fffffffu);
     fx_sample(fx_pair(lo, hi), emax, *h, *l);
   }
-  __device__ __forceinline__ bool fit() const { return (int)(over >> 20) <= emax; }
+  __device__ __forceinline__ bool fit() const { return (int)((over + 1) >> 20) <= emax; }
   template <bool FULL>
   __device__ __forceinline__ bool scale() {
     constexpr int A = FULL ? 0 : 1, B = FULL ? 4 : 3;

@@ -21,6 +21,11 @@
 
 namespace arb {
 
+// Bound by the IMAD.WIDE pipe (4 cycles a warp instruction and scheduler; 'both'
+// takes 1332 of them a query, 61 % of its cycles at 305 queries a bin) and by the
+// dependent issue of its chains at 12 to 16 warps per SM.  Three CTAs of 128
+// threads and 168 registers for 'both' (four of 128 with spills 3418 against 3276 us
+// for the binned pass of 1e7 on 256^3; 96, 160, 192 or 256 threads 3447-3636).
 constexpr int FX_THREADS = 128;
 constexpr int FX_EVEN3 = 5, FX_EVEN4 = 5;
 
@@ -107,7 +112,7 @@ struct FxRawSrc3 {
   __device__ __forceinline__ bool fit() const {
     bool ok = true;
 #pragma unroll
-    for (int f = 0; f < F; ++f) ok &= (int)(over[f] >> 20) <= emax[f];
+    for (int f = 0; f < F; ++f) ok &= (int)((over[f] + 1) >> 20) <= emax[f];
     return ok;
   }
   __device__ __forceinline__ bool scale() {
@@ -173,14 +178,14 @@ __device__ __forceinline__ uint32_t fx_bits_at(const uint32_t *w, int o) {
 }
 
 template <int F>
-__global__ void __launch_bounds__(FX_THREADS, 4) eval_fx3_kernel(arb_grid g, KParams kp, BinGeom bg,
+__global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(arb_grid g, KParams kp, BinGeom bg,
                                                                               int64_t nq, arb_query_out o,
                                                                               SortedWork w) {
   extern __shared__ __align__(16) unsigned char fx_smem[];
   FxTile3<F> &tile = *reinterpret_cast<FxTile3<F> *>(fx_smem);
   __shared__ FxTileMax<F> smax;
   __shared__ uint32_t large_bits[F][(TILE_PTS + FX_THREADS) / 32 + 1];
-  const QRec<double> *recs = reinterpret_cast<const QRec<double> *>(w.rec);
+  const QRec64<3> *recs = reinterpret_cast<const QRec64<3> *>(w.rec);
   const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2];
   const int cls = bg.cls;
   int turn = 0;
@@ -271,17 +276,17 @@ __global__ void __launch_bounds__(FX_THREADS, 4) eval_fx3_kernel(arb_grid g, KPa
     // warps start at another quarter of the records in each bin: the last,
     // partial round of a bin would otherwise always fall to the same warps, and
     // warp w of every CTA runs on scheduler w
-    const uint32_t first = t0 + ((threadIdx.x + FX_THREADS / 4 * (uint32_t)turn) & (FX_THREADS - 1));
+    const uint32_t first = t0 + ((threadIdx.x + 32u * (uint32_t)turn) % FX_THREADS);
     ++turn;
     // the next record is loaded while this one is evaluated
-    QRec<double> next;
+    QRec64<3> next;
     if (first < t1) next = recs[first];
     for (uint32_t t = first; t < t1; t += FX_THREADS) {
-      const QRec<double> q = next;
+      const QRec64<3> q = next;
       if (t + FX_THREADS < t1) next = recs[t + FX_THREADS];
       int64_t c[3];
-      unpack_cell<3>(q.cell, c);
-      const double fr[3] = {q.f[0], q.f[1], q.f[2]};
+      cell_coords<3>((int64_t)rec64_cell<3>(q), g, c);
+      const double fr[3] = {rec64_frac<3>(q, 0), rec64_frac<3>(q, 1), rec64_frac<3>(q, 2)};
       double val[F], grad[3] = {0.0, 0.0, 0.0};
       const int base = (((int)c[2] - og[2]) * TILE_EDGE + ((int)c[1] - og[1])) * TILE_EDGE + ((int)c[0] - og[0]);
       bool fine = ok;
@@ -316,8 +321,8 @@ __global__ void __launch_bounds__(FX_THREADS, 4) eval_fx3_kernel(arb_grid g, KPa
   // records that need no evaluation (out of volume, NaN, sentinel column)
   for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const QRec<double> q = recs[t];
-    write_const<3, F>(o, q.row, (q.cell & 1ULL) && !g.sentinel_nan ? 0.0 : qnan());
+    const QRec64<3> q = recs[t];
+    write_const<3, F>(o, q.row, rec64_cell<3>(q) != NAN_CELL<3> && !g.sentinel_nan ? 0.0 : qnan());
   }
 }
 
@@ -328,6 +333,7 @@ struct FxTile4 {
 };
 
 struct FxTileSrc4 {
+  static constexpr int UNROLL = 4;
   const int2 *v;
   int base;
   __device__ __forceinline__ int at(int j, int k, int t) const {
@@ -341,6 +347,7 @@ struct FxTileSrc4 {
 };
 
 struct FxRawSrc4 {
+  static constexpr int UNROLL = 1;
   const int2 *v;
   int base;
   int emax;
@@ -353,7 +360,7 @@ struct FxRawSrc4 {
     over = max(over, (uint32_t)u.x & 0x7fffffffu);
     fx_sample(fx_pair((uint32_t)u.y, (uint32_t)u.x), emax, *h, *l);
   }
-  __device__ __forceinline__ bool fit() const { return (int)(over >> 20) <= emax; }
+  __device__ __forceinline__ bool fit() const { return (int)((over + 1) >> 20) <= emax; }
   __device__ __forceinline__ bool scale() {
     FxMax m;
 #pragma unroll
@@ -369,13 +376,13 @@ struct FxRawSrc4 {
 };
 
 template <int F>
-__global__ void __launch_bounds__(FX_THREADS, 3) eval_fx4_kernel(arb_grid g, KParams kp, BinGeom bg, int64_t nq,
+__global__ void __launch_bounds__(FX_THREADS, F == 1 ? 3 : 2) eval_fx4_kernel(arb_grid g, KParams kp, BinGeom bg, int64_t nq,
                                                                  arb_query_out o, SortedWork w) {
   extern __shared__ __align__(16) unsigned char fx_smem[];
   FxTile4<F> &tile = *reinterpret_cast<FxTile4<F> *>(fx_smem);
   __shared__ FxTileMax<F> smax;
   __shared__ uint32_t large_bits[F][(TILE4_PTS + 31) / 32 + 1];
-  const QRec<double> *recs = reinterpret_cast<const QRec<double> *>(w.rec);
+  const QRec64<4> *recs = reinterpret_cast<const QRec64<4> *>(w.rec);
   const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2], nt = g.n[3];
   const int cls = bg.cls;
   int turn = 0;
@@ -449,13 +456,13 @@ __global__ void __launch_bounds__(FX_THREADS, 3) eval_fx4_kernel(arb_grid g, KPa
         }
     }
     __syncthreads();
-    const uint32_t first = t0 + ((threadIdx.x + FX_THREADS / 4 * (uint32_t)turn) & (FX_THREADS - 1));
+    const uint32_t first = t0 + ((threadIdx.x + 32u * (uint32_t)turn) % FX_THREADS);
     ++turn;
     for (uint32_t t = first; t < t1; t += FX_THREADS) {
-      const QRec<double> q = recs[t];
+      const QRec64<4> q = recs[t];
       int64_t c[4];
-      unpack_cell<4>(q.cell, c);
-      const double fr[4] = {q.f[0], q.f[1], q.f[2], q.f[3]};
+      cell_coords<4>((int64_t)rec64_cell<4>(q), g, c);
+      const double fr[4] = {rec64_frac<4>(q, 0), rec64_frac<4>(q, 1), rec64_frac<4>(q, 2), rec64_frac<4>(q, 3)};
       double val[F], grad[4] = {0.0, 0.0, 0.0, 0.0};
       FxW wt[4];
 #pragma unroll
@@ -511,8 +518,8 @@ __global__ void __launch_bounds__(FX_THREADS, 3) eval_fx4_kernel(arb_grid g, KPa
   }
   for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const QRec<double> q = recs[t];
-    write_const<4, F>(o, q.row, (q.cell & 1ULL) && !g.sentinel_nan ? 0.0 : qnan());
+    const QRec64<4> q = recs[t];
+    write_const<4, F>(o, q.row, rec64_cell<4>(q) != NAN_CELL<4> && !g.sentinel_nan ? 0.0 : qnan());
   }
 }
 
@@ -552,16 +559,15 @@ static bool launch_eval_fx_f(const arb_grid *g, const KParams &kp, const BinGeom
 // Launches the bin-staged float64 kernel when it applies (bins of the tile's
 // shape with bank classes, and enough queries); returns false otherwise.
 // A tile costs its bin 5.4e3 (F = 4) conversions however many queries it has;
-// below the line the queries are evaluated in bin order from the grid
-// (eval_sorted_kernel).  Whole passes, tile against that: 'both' 256^3 at 30
-// queries a bin 1308 : 590 us and at 305 3710 : 4988 us; norm 128^3 at 244 219 : 236
+// below the line (fx_dense) the queries are evaluated in bin order from the
+// grid (eval_sorted_kernel).  Whole passes, tile against that: 'both' 256^3 at 30
+// queries a bin 1308 : 590 us and at 305 3276 : 4613 us; norm 128^3 at 244 219 : 236
 // and at 122 145 : 134; vector 128^3 at 49 125 : 115 and at 244 252 : 377; 4D
-// scalar at 89 294 : 272 and at 670 1157 : 1735.
+// scalar at 89 294 : 272 and at 670 1130 : 1701.
 template <int DIM>
 static bool launch_eval_fx(const arb_grid *g, const KParams &kp, const BinGeom &bg, int64_t nq,
                            const arb_query_out *out, const SortedWork &w, cudaStream_t s) {
-  if (bg.cls != 4 || bg.shift != (DIM == 3 ? 3 : 2)) return false;
-  if (nq < (DIM == 3 && g->nfield == 3 ? 64 : 128) * bg.nbins) return false;
+  if (bg.cls != 4) return false;
   switch (g->nfield) {
     case 1: return launch_eval_fx_f<DIM, 1>(g, kp, bg, nq, out, w, s);
     case 3: return launch_eval_fx_f<DIM, 3>(g, kp, bg, nq, out, w, s);

@@ -32,26 +32,77 @@
 
 namespace arb {
 
-// Bin-ordered query record: packed cell (or CELL_SPECIAL | code), the
-// query's row and its fractional offsets (float32 in mixed precision: 32
-// bytes, one sector; float64: 48 bytes).
-template <typename T>
-struct QRec;
-template <>
-struct __align__(32) QRec<float> {
+// Bin-ordered query records.  Mixed precision: packed cell (or CELL_SPECIAL |
+// code), the query's row and its fractional offsets in float32, 32 bytes (one
+// sector).  Float64: the flat cell index, the row and the float64 fractions in
+// 32 bytes (3D) or 40 (4D); a fraction in [0, 1) leaves bits 62 and 63 of its
+// float64 clear, and they hold the index' bits from 32 up.
+struct __align__(32) QRec {
   unsigned long long cell;
   uint32_t row;
   float f[4];
   uint32_t pad;
 };
-template <>
-struct __align__(16) QRec<double> {
-  unsigned long long cell;
-  uint32_t row;
-  uint32_t pad;
-  double f[4];
+template <int DIM>
+struct __align__(DIM == 3 ? 32 : 8) QRec64 {
+  uint32_t cell, row;
+  unsigned long long f[DIM];
 };
-static_assert(sizeof(QRec<float>) == 32 && sizeof(QRec<double>) == 48, "record sizes");
+static_assert(sizeof(QRec) == 32 && sizeof(QRec64<3>) == 32 && sizeof(QRec64<4>) == 40, "record sizes");
+
+// Index of a float64 record that needs no evaluation: NaN_CELL (out of volume
+// or a NaN row), NaN_CELL - 1 (the reference's sentinel column).
+template <int DIM>
+constexpr unsigned long long NAN_CELL = (1ULL << (32 + 2 * DIM)) - 1ULL;
+
+template <int DIM>
+__device__ __forceinline__ QRec64<DIM> make_rec64(unsigned long long cell, uint32_t row, const double frac[DIM]) {
+  QRec64<DIM> r;
+  r.cell = (uint32_t)cell;
+  r.row = row;
+#pragma unroll
+  for (int a = 0; a < DIM; ++a)
+    r.f[a] = (unsigned long long)__double_as_longlong(frac[a]) | (cell >> (32 + 2 * a) & 3ULL) << 62;
+  return r;
+}
+template <int DIM>
+__device__ __forceinline__ unsigned long long rec64_cell(const QRec64<DIM> &r) {
+  unsigned long long c = r.cell;
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) c |= (r.f[a] >> 62) << (32 + 2 * a);
+  return c;
+}
+template <int DIM>
+__device__ __forceinline__ double rec64_frac(const QRec64<DIM> &r, int a) {
+  return __longlong_as_double((long long)(r.f[a] & 0x3fffffffffffffffULL));
+}
+
+// Record t as the evaluators take it: row, cell coordinates and fractions;
+// false for a row that needs no evaluation (sentinel: its output is the
+// reference's sentinel column, otherwise NaN).
+template <int DIM, typename T>
+__device__ __forceinline__ bool read_rec(const void *recs, int64_t t, const arb_grid &g, int64_t &row, int64_t c[DIM],
+                                         T f[DIM], bool &sentinel) {
+  if constexpr (sizeof(T) == 4) {
+    const QRec r = reinterpret_cast<const QRec *>(recs)[t];
+    row = r.row;
+    sentinel = r.cell & 1ULL;
+    if (r.cell & CELL_SPECIAL) return false;
+    unpack_cell<DIM>(r.cell, c);
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) f[a] = r.f[a];
+  } else {
+    const QRec64<DIM> r = reinterpret_cast<const QRec64<DIM> *>(recs)[t];
+    const unsigned long long cell = rec64_cell<DIM>(r);
+    row = r.row;
+    sentinel = cell == NAN_CELL<DIM> - 1;
+    if (cell >= NAN_CELL<DIM> - 1) return false;
+    cell_coords<DIM>((int64_t)cell, g, c);
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) f[a] = rec64_frac<DIM>(r, a);
+  }
+  return true;
+}
 
 // Placement header of a bin with 16 bank classes: where its records start
 // and how many each class holds, so the placement pass reads one sector
@@ -70,7 +121,7 @@ struct SortedWork {
                     // the special sub-bin nsub [offs[nsub], nq)
   uint32_t *part;   // per-block totals of the scan
   BinHdr *hdr;      // nbins placement headers (bins with bank classes; null otherwise)
-  void *rec;        // nq records (QRec<float> or QRec<double>) in bin order; with bank classes each
+  void *rec;        // nq records (QRec, QRec64<3> or QRec64<4>) in bin order; with bank classes each
                     // bin's records are in its bank schedule (see bank_slot)
 };
 
@@ -78,8 +129,9 @@ struct BinGeom {
   int64_t nb[4];     // bins per axis
   int64_t nbins;     // product
   int shift;         // log2 cells per bin edge
-  int cls;           // log2 bank classes per bin (4: 3D 8^3-cell bins and 4D 4^4-cell bins, in mixed
-                     // precision of scalar fields only; 0 otherwise)
+  int cls;           // log2 bank classes per bin (4 where the bins are staged in shared memory: 3D mixed
+                     // 8^3-cell bins, 4D mixed scalar 4^4-cell bins, and both shapes in float64 when
+                     // the queries are dense; 0 otherwise)
   int64_t nsub;      // nbins << cls sub-bins (bin-major); the special sub-bin is index nsub
 };
 
@@ -103,7 +155,12 @@ __host__ __device__ __forceinline__ int bank_class4(int64_t cx, int64_t cy, int6
   return (int)((cx + 7 * cy + cz + 7 * ct) & 15);
 }
 
-static inline BinGeom bin_geom(const arb_grid *g, int precision) {
+// Float64 bins with enough queries to be staged (see launch_eval_fx).
+static inline bool fx_dense(const arb_grid *g, int64_t nbins, int64_t nq) {
+  return nq >= (g->dim == 3 && g->nfield == 3 ? 64 : 128) * nbins;
+}
+
+static inline BinGeom bin_geom(const arb_grid *g, int precision, int64_t nq) {
   BinGeom b;
   b.shift = (g->bin_shift > 0 && g->bin_shift <= 8) ? g->bin_shift : (g->dim == 3 ? 3 : 2);
   b.nbins = 1;
@@ -117,8 +174,12 @@ static inline BinGeom bin_geom(const arb_grid *g, int precision) {
     b.nbins *= b.nb[a];
   }
   b.cls = 0;
-  if (g->dim == 3 && b.shift == 3) b.cls = 4;
-  if (g->dim == 4 && b.shift == 2 && (g->nfield == 1 || precision != ARB_PREC_MIXED)) b.cls = 4;
+  if (precision == ARB_PREC_MIXED) {
+    if (g->dim == 3 && b.shift == 3) b.cls = 4;
+    if (g->dim == 4 && b.shift == 2 && g->nfield == 1) b.cls = 4;
+  } else if (b.shift == (g->dim == 3 ? 3 : 2) && fx_dense(g, b.nbins, nq)) {
+    b.cls = 4;
+  }
   b.nsub = b.nbins << b.cls;
   return b;
 }
@@ -133,8 +194,8 @@ constexpr int64_t SCAN_CHUNK = (int64_t)SCAN_THREADS * SCAN_PER;
 static inline int64_t scan_blocks(int64_t n) { return (n + SCAN_CHUNK - 1) / SCAN_CHUNK; }
 
 static size_t carve(SortedWork *w, void *base, const arb_grid *g, int precision, int64_t nq) {
-  const BinGeom bg = bin_geom(g, precision);
-  const size_t tsz = precision == ARB_PREC_MIXED ? 4 : 8;
+  const BinGeom bg = bin_geom(g, precision, nq);
+  const bool mixed = precision == ARB_PREC_MIXED;
   size_t off = 0;
   char *p = (char *)base;
   auto take = [&](size_t bytes) {
@@ -147,9 +208,15 @@ static size_t carve(SortedWork *w, void *base, const arb_grid *g, int precision,
   t.offs = (uint32_t *)take(sizeof(uint32_t) * (bg.nsub + 1));
   t.part = (uint32_t *)take(sizeof(uint32_t) * scan_blocks(bg.nsub + 1));
   t.hdr = bg.cls ? (BinHdr *)take(sizeof(BinHdr) * bg.nbins) : nullptr;
-  t.rec = take((tsz == 4 ? sizeof(QRec<float>) : sizeof(QRec<double>)) * nq);
+  t.rec = take((mixed ? sizeof(QRec) : g->dim == 3 ? sizeof(QRec64<3>) : sizeof(QRec64<4>)) * nq);
   if (w) *w = t;
-  return off;
+  if (mixed) return off;
+  // The stated need of a float64 call is 48 bytes a row and one counter pair a
+  // bin, so row limits do not move with the layout.  It is enough: classes take
+  // 152 bytes a bin more, at 64 rows a bin or more, and a row 8 or 16 bytes less.
+  const size_t stated = 2 * align_up(sizeof(uint32_t) * (bg.nbins + 1)) +
+                        align_up(sizeof(uint32_t) * scan_blocks(bg.nbins + 1)) + align_up(48 * nq);
+  return off > stated ? off : stated;
 }
 
 // Coordinate step of query row i: cell index, fraction, packed cell word
@@ -241,6 +308,14 @@ __device__ __forceinline__ uint32_t bank_slot_hdr(const uint32_t cnt[4], uint32_
   return pos;
 }
 
+// One 32-byte store: a whole sector, no partial-sector merge in L2.
+__device__ __forceinline__ void store_rec32(void *dst, const void *rec) {
+  const uint32_t *u = reinterpret_cast<const uint32_t *>(rec);
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(u[0]), "r"(u[1]), "r"(u[2]),
+               "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7])
+               : "memory");
+}
+
 template <int DIM, bool EXACT, typename T>
 __global__ void __launch_bounds__(256) bin_place_kernel(arb_grid g, KParams kp, BinGeom bg, const double *q,
                                                         int64_t nq, int64_t qs, SortedWork w) {
@@ -250,7 +325,7 @@ __global__ void __launch_bounds__(256) bin_place_kernel(arb_grid g, KParams kp, 
   unsigned long long cw;
   int64_t bin;
   bool bad;
-  (void)bin_step<DIM, EXACT, T>(g, kp, bg, q + i * qs, frac, cw, bin, bad);
+  const CoordStep s = bin_step<DIM, EXACT, T>(g, kp, bg, q + i * qs, frac, cw, bin, bad);
   // rank inside the sub-bin (any order: the count runs back down to zero)
   const uint32_t r = atomicSub(&w.hist[bin], 1u) - 1u;
   uint32_t pos;
@@ -272,20 +347,26 @@ __global__ void __launch_bounds__(256) bin_place_kernel(arb_grid g, KParams kp, 
   } else {
     pos = w.offs[bin] + r;
   }
-  QRec<T> rec;
-  rec.cell = cw;
-  rec.row = (uint32_t)i;
-#pragma unroll
-  for (int a = 0; a < 4; ++a) rec.f[a] = a < DIM ? frac[a] : T(0);
-  rec.pad = 0;
   if constexpr (sizeof(T) == 4) {
-    // one 32-byte store: a whole sector, no partial-sector merge in L2
-    const uint32_t *u = reinterpret_cast<const uint32_t *>(&rec);
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(reinterpret_cast<QRec<T> *>(w.rec) + pos),
-                 "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7])
-                 : "memory");
+    QRec rec;
+    rec.cell = cw;
+    rec.row = (uint32_t)i;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) rec.f[a] = a < DIM ? frac[a] : 0.f;
+    rec.pad = 0;
+    store_rec32(reinterpret_cast<QRec *>(w.rec) + pos, &rec);
   } else {
-    reinterpret_cast<QRec<T> *>(w.rec)[pos] = rec;
+    const unsigned long long cell =
+        (cw & CELL_SPECIAL) ? NAN_CELL<DIM> - (cw & 1ULL) : (unsigned long long)s.idx;
+#pragma unroll
+    for (int a = 0; a < DIM; ++a)
+      if (cw & CELL_SPECIAL) frac[a] = 0.0;
+    const QRec64<DIM> rec = make_rec64<DIM>(cell, (uint32_t)i, frac);
+    QRec64<DIM> *dst = reinterpret_cast<QRec64<DIM> *>(w.rec) + pos;
+    if constexpr (DIM == 3)
+      store_rec32(dst, &rec);
+    else
+      *dst = rec;
   }
 }
 
@@ -394,18 +475,13 @@ __global__ void __launch_bounds__(DIM == 3 ? 256 : 128, MIXED ? 1 : (DIM == 3 ? 
   using T = typename std::conditional<MIXED, float, double>::type;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= nq) return;
-  const QRec<T> r = reinterpret_cast<const QRec<T> *>(w.rec)[t];
-  const unsigned long long cw = r.cell;
-  const int64_t i = r.row;
-  if (cw & CELL_SPECIAL) {
-    write_const<DIM, F>(o, i, (cw & 1ULL) && !g.sentinel_nan ? 0.0 : qnan());
+  int64_t i, c[DIM];
+  T fr[DIM];
+  bool sentinel;
+  if (!read_rec<DIM, T>(w.rec, t, g, i, c, fr, sentinel)) {
+    write_const<DIM, F>(o, i, sentinel && !g.sentinel_nan ? 0.0 : qnan());
     return;
   }
-  int64_t c[DIM];
-  unpack_cell<DIM>(cw, c);
-  T fr[DIM];
-#pragma unroll
-  for (int a = 0; a < DIM; ++a) fr[a] = r.f[a];
   double val[F], grad[DIM];
 #pragma unroll
   for (int a = 0; a < DIM; ++a) grad[a] = 0.0;
@@ -548,7 +624,7 @@ __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) e
   extern __shared__ __align__(16) unsigned char binc_smem[];
   BinTile<F> *tiles = reinterpret_cast<BinTile<F> *>(binc_smem);
   const int64_t nbins = bg.nbins;
-  const QRec<float> *recs = reinterpret_cast<const QRec<float> *>(w.rec);
+  const QRec *recs = reinterpret_cast<const QRec *>(w.rec);
   // bin b holds records [offs[16 b], offs[16 b + 16]) (its 16 class sub-bins)
   const int cls = bg.cls;
   auto begin = [&](int64_t bb) { return w.offs[bb << cls]; };
@@ -580,10 +656,10 @@ __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) e
     if (t1 > t0) {
       origin(b, og);
       // the next record is loaded while this one is evaluated
-      QRec<float> rnext;
+      QRec rnext;
       if (t0 + threadIdx.x < t1) rnext = recs[t0 + threadIdx.x];
       for (uint32_t t = t0 + threadIdx.x; t < t1; t += BINC_THREADS) {
-        const QRec<float> r = rnext;
+        const QRec r = rnext;
         if (t + BINC_THREADS < t1) rnext = recs[t + BINC_THREADS];
         int64_t c[3];
         unpack_cell<3>(r.cell, c);
@@ -613,7 +689,7 @@ __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) e
   // records that need no evaluation (out of volume, NaN, sentinel column)
   for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const QRec<float> r = recs[t];
+    const QRec r = recs[t];
     write_const<3, F>(o, r.row, (r.cell & 1ULL) && !g.sentinel_nan ? 0.0 : qnan());
   }
 }
@@ -724,7 +800,7 @@ __global__ void __launch_bounds__(BIN4_THREADS) eval_bin4_kernel(arb_grid g, KPa
   extern __shared__ __align__(16) unsigned char bin4_smem[];
   BinTile4 *tiles = reinterpret_cast<BinTile4 *>(bin4_smem);
   const int64_t nbins = bg.nbins;
-  const QRec<float> *recs = reinterpret_cast<const QRec<float> *>(w.rec);
+  const QRec *recs = reinterpret_cast<const QRec *>(w.rec);
   int stage = 0;
   int64_t b = blockIdx.x;
   // bin b holds records [offs[b << cls], offs[(b + 1) << cls]) (its class
@@ -745,7 +821,7 @@ __global__ void __launch_bounds__(BIN4_THREADS) eval_bin4_kernel(arb_grid g, KPa
       int64_t og[4];
       bin_origin4(b, bg, og);
       for (int64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
-        const QRec<float> r = recs[t];
+        const QRec r = recs[t];
         int64_t c[4];
         unpack_cell<4>(r.cell, c);
         TileBlock4 blk;
@@ -765,7 +841,7 @@ __global__ void __launch_bounds__(BIN4_THREADS) eval_bin4_kernel(arb_grid g, KPa
   // records that need no evaluation (out of volume, NaN, sentinel column)
   for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
        t += (int64_t)gridDim.x * blockDim.x) {
-    const QRec<float> r = recs[t];
+    const QRec r = recs[t];
     write_const<4, 1>(o, r.row, (r.cell & 1ULL) && !g.sentinel_nan ? 0.0 : qnan());
   }
 }
@@ -838,16 +914,14 @@ __global__ void __launch_bounds__(256) eval_tab_coop_kernel(arb_grid g, KParams 
   const T *tab = reinterpret_cast<const T *>(g.table);
   const int ey = j & 3, jz = j >> 2;
   for (int64_t t = t0 + (threadIdx.x >> 3); t < t1; t += blockDim.x >> 3) {
-    const QRec<T> r = reinterpret_cast<const QRec<T> *>(w.rec)[t];
-    const unsigned long long cw = r.cell;
-    const int64_t i = r.row;
-    if (cw & CELL_SPECIAL) {
-      if (j == 0) write_const<DIM, F>(o, i, (cw & 1ULL) && !g.sentinel_nan ? 0.0 : qnan());
+    int64_t i, c[DIM];
+    T fr[DIM];
+    bool sentinel;
+    if (!read_rec<DIM, T>(w.rec, t, g, i, c, fr, sentinel)) {
+      if (j == 0) write_const<DIM, F>(o, i, sentinel && !g.sentinel_nan ? 0.0 : qnan());
       continue;
     }
-    int64_t c[DIM];
-    unpack_cell<DIM>(cw, c);
-    const T x = r.f[0], y = r.f[1], z = r.f[2];
+    const T x = fr[0], y = fr[1], z = fr[2];
     // y^ey, z^jz, z^(jz+2) and their derivatives: selects, not indexing
     const T y2 = y * y, z2 = z * z;
     const T wy = ey == 0 ? T(1) : ey == 1 ? y : ey == 2 ? y2 : y2 * y;
@@ -856,7 +930,7 @@ __global__ void __launch_bounds__(256) eval_tab_coop_kernel(arb_grid g, KParams 
     const T dwza = jz ? T(1) : T(0), dwzb = jz ? T(3) * z2 : T(2) * z;
     T wt[4] = {T(1), T(1), T(1), T(1)}, dwt[4] = {T(0), T(0), T(0), T(0)};
     if constexpr (DIM == 4) {
-      const T u = r.f[3], u2 = u * u;
+      const T u = fr[3], u2 = u * u;
       wt[1] = u;
       wt[2] = u2;
       wt[3] = u2 * u;
@@ -922,7 +996,7 @@ __global__ void __launch_bounds__(256) eval_tab_coop_kernel(arb_grid g, KParams 
 template <int DIM, bool MIXED>
 static void launch_eval(const arb_grid *g, const KParams &kp, int64_t nq, const arb_query_out *out,
                         const SortedWork &w, bool table, cudaStream_t s) {
-  const BinGeom bg = bin_geom(g, MIXED ? ARB_PREC_MIXED : ARB_PREC_FP64);
+  const BinGeom bg = bin_geom(g, MIXED ? ARB_PREC_MIXED : ARB_PREC_FP64, nq);
   if (DIM == 3 && MIXED && !table && launch_eval_binc(g, kp, bg, nq, out, w, s)) return;
   if (DIM == 4 && MIXED && !table && launch_eval_bin4(g, kp, bg, nq, out, w, s)) return;
   if (!MIXED && !table && launch_eval_fx<DIM>(g, kp, bg, nq, out, w, s)) return;
@@ -958,7 +1032,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) adjoint_bin_kernel(arb_grid g, KP
   BinTile<1> *tiles = reinterpret_cast<BinTile<1> *>(adj_smem);
   float *gt = reinterpret_cast<float *>(adj_smem + 2 * sizeof(BinTile<1>));  // dL/df of the bin's points
   const int64_t nbins = bg.nbins;
-  const QRec<float> *recs = reinterpret_cast<const QRec<float> *>(w.rec);
+  const QRec *recs = reinterpret_cast<const QRec *>(w.rec);
   const int cls = bg.cls;
   auto begin = [&](int64_t bb) { return w.offs[bb << cls]; };
   auto count = [&](int64_t bb) { return bb < nbins ? w.offs[(bb + 1) << cls] - begin(bb) : 0u; };
@@ -993,7 +1067,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) adjoint_bin_kernel(arb_grid g, KP
       origin(b, og);
       const float2 *tv = tiles[stage].v;
       for (uint32_t t = t0 + threadIdx.x; t < t1; t += ADJ_THREADS) {
-        const QRec<float> r = recs[t];
+        const QRec r = recs[t];
         const int64_t row = r.row;
         const float dv = dval ? (float)dval[row] : 0.f;
         float dg[3] = {0.f, 0.f, 0.f};
@@ -1162,6 +1236,7 @@ extern "C" int arb_query_eval_sorted(const arb_grid *g, int32_t precision, int32
   const int bits = g->dim == 3 ? cell_bits<3>() : cell_bits<4>();
   for (int a = 0; a < g->dim; ++a)
     if (g->n[a] - 3 >= ((int64_t)1 << bits)) return ARB_ERR_UNSUPPORTED;  // cells per axis
+  if (g->nc >= (int64_t)1 << 37) return ARB_ERR_UNSUPPORTED;  // float64 records (a grid of 1 TB)
   const bool mixed = precision == ARB_PREC_MIXED;
   if (use_table) {
     if (!g->table || g->table_prec != precision) return ARB_ERR_INVALID;
@@ -1170,7 +1245,7 @@ extern "C" int arb_query_eval_sorted(const arb_grid *g, int32_t precision, int32
   }
   SortedWork w;
   if (carve(&w, work, g, precision, nq) > work_bytes) return ARB_ERR_INVALID;
-  const BinGeom bg = bin_geom(g, precision);
+  const BinGeom bg = bin_geom(g, precision, nq);
   cudaStream_t s = (cudaStream_t)stream;
   const arb_query_out out_norm = normalize_out(*out, g->dim);
   out = &out_norm;
@@ -1210,9 +1285,10 @@ extern "C" int arb_query_bin(const arb_grid *g, int32_t precision, double *q, in
   const int bits = g->dim == 3 ? cell_bits<3>() : cell_bits<4>();
   for (int a = 0; a < g->dim; ++a)
     if (g->n[a] - 3 >= ((int64_t)1 << bits)) return ARB_ERR_UNSUPPORTED;
+  if (g->nc >= (int64_t)1 << 37) return ARB_ERR_UNSUPPORTED;
   SortedWork w;
   if (carve(&w, work, g, precision, nq) > work_bytes) return ARB_ERR_INVALID;
-  const BinGeom bg = bin_geom(g, precision);
+  const BinGeom bg = bin_geom(g, precision, nq);
   cudaStream_t s = (cudaStream_t)stream;
   const arb_query_out out_norm = normalize_out(*out, g->dim);
   out = &out_norm;
@@ -1302,7 +1378,7 @@ extern "C" int arb_adjoint_binned(const arb_grid *g, int32_t precision, const do
   gb.bin_shift = 3;  // 8^3-cell bins: the staged tiles' shape
   SortedWork w;
   if (carve(&w, work, &gb, precision, nq) > work_bytes) return ARB_ERR_INVALID;
-  const BinGeom bg = bin_geom(&gb, precision);
+  const BinGeom bg = bin_geom(&gb, precision, nq);
   cudaStream_t s = (cudaStream_t)stream;
   arb_query_out none{};
   const arb_query_out out = normalize_out(none, 3);
