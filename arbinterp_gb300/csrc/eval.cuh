@@ -140,9 +140,9 @@ __device__ __forceinline__ bool query_prologue(const arb_grid &g, const KParams 
 
 // ---- row loaders ------------------------------------------------------------
 // 4 consecutive grid points x F fields starting at flat point p.
-template <int F>
+template <int F, int STEP>
 __device__ __forceinline__ void load_row64(const double *grid, int64_t p, double v[4][F]) {
-  const double *r = grid + p * F;
+  const double *r = grid + p * STEP;
   if (F == 4) {
     const double2 *r2 = reinterpret_cast<const double2 *>(r);
 #pragma unroll
@@ -157,7 +157,7 @@ __device__ __forceinline__ void load_row64(const double *grid, int64_t p, double
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int f = 0; f < F; ++f) v[i][f] = __ldg(r + i * F + f);
+      for (int f = 0; f < F; ++f) v[i][f] = __ldg(r + i * STEP + f);
   }
 }
 
@@ -190,6 +190,18 @@ struct Grid32Block3 {  // the mixed grid in global memory
   template <int F>
   __device__ __forceinline__ void load(int64_t p, int f, float &h, float &l) const {
     g32_load<F>(g32, npts, p, f, h, l);
+  }
+};
+
+// |B| alone of a 'both' grid as (hi, lo) pairs (norm_pairs_kernel).
+struct NormBlock3 {
+  const float2 *v;
+  int64_t sy, sz, base;
+  __device__ __forceinline__ int64_t at(int i, int j, int k) const { return base + k * sz + j * sy + i; }
+  __device__ __forceinline__ float4 hi4(int64_t p) const { return make_float4(0.f, 0.f, 0.f, __ldg(v + p).x); }
+  __device__ __forceinline__ void lo_row(int64_t p, float l[4]) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) l[i] = __ldg(v + p + i).y;
   }
 };
 
@@ -505,7 +517,7 @@ struct EvalOut {
   double val[F], grad[N];
 };
 
-template <int F>
+template <int F, int STEP>
 static __device__ __noinline__ EvalOut<F, 3> eval_otf3_f64(const double *grid, int64_t nx, int64_t ny, EvalArgs<3> in) {
   constexpr bool GRAD = (F != 3);
   double wx[4], wy[4], wz[4], dx[4], dy[4], dz[4];
@@ -528,7 +540,7 @@ static __device__ __noinline__ EvalOut<F, 3> eval_otf3_f64(const double *grid, i
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       double v[4][F];
-      load_row64<F>(grid, ((in.c[2] + k) * ny + (in.c[1] + j)) * nx + in.c[0], v);
+      load_row64<F, STEP>(grid, ((in.c[2] + k) * ny + (in.c[1] + j)) * nx + in.c[0], v);
       double ax[F];
 #pragma unroll
       for (int f = 0; f < F; ++f)
@@ -563,13 +575,13 @@ static __device__ __noinline__ EvalOut<F, 3> eval_otf3_f64(const double *grid, i
 
 // The block as a whole sets the scale: blocks with a sample far above the
 // query's own cell, or float64 arithmetic where the scaling does not hold.
-template <int F>
+template <int F, int STEP>
 static __device__ __noinline__ EvalOut<F, 3> eval_otf3_full(const double *grid, int64_t nx, int64_t ny, EvalArgs<3> in) {
-  FxGrid3<F> src;
-  src.p = grid + ((in.c[2] * ny + in.c[1]) * nx + in.c[0]) * F;
-  src.sy = nx * F;
-  src.sz = nx * ny * F;
-  if (!src.template scale<true>()) return eval_otf3_f64<F>(grid, nx, ny, in);
+  FxGrid3<F, STEP> src;
+  src.p = grid + ((in.c[2] * ny + in.c[1]) * nx + in.c[0]) * STEP;
+  src.sy = nx * STEP;
+  src.sz = nx * ny * STEP;
+  if (!src.template scale<true>()) return eval_otf3_f64<F, STEP>(grid, nx, ny, in);
   FxW wx, wy, wz;
   fx_axis<1>(fx_bits(in.frac[0]), wx);
   fx_axis<1>(fx_bits(in.frac[1]), wy);
@@ -582,7 +594,7 @@ static __device__ __noinline__ EvalOut<F, 3> eval_otf3_full(const double *grid, 
   return o;
 }
 
-template <int F>
+template <int F, int STEP = F>
 __device__ __forceinline__ void eval_otf3_slow(const arb_grid &g, const KParams &kp, const int64_t c[3],
                                                const double frac[3], double val[F], double grad[3]) {
   EvalArgs<3> in;
@@ -592,7 +604,7 @@ __device__ __forceinline__ void eval_otf3_slow(const arb_grid &g, const KParams 
     in.frac[a] = frac[a];
     in.inv_h[a] = kp.inv_h[a];
   }
-  const EvalOut<F, 3> o = eval_otf3_full<F>(g.grid64, g.n[0], g.n[1], in);
+  const EvalOut<F, 3> o = eval_otf3_full<F, STEP>(g.grid64 + (STEP - F), g.n[0], g.n[1], in);
 #pragma unroll
   for (int f = 0; f < F; ++f) val[f] = o.val[f];
   if (F != 3) {
@@ -605,14 +617,15 @@ __device__ __forceinline__ void eval_otf3_slow(const arb_grid &g, const KParams 
 // bound by L1 wavefronts and the conversions (~20 integer operations a sample).
 // 1e5 scalar queries on 41^3: 64 -> 31 us; RK4, the batched launch and sparse
 // bin-ordered queries take it too.
-template <int F>
+// STEP = 4 with F = 1: |B| alone of a 'both' grid.
+template <int F, int STEP = F>
 __device__ __forceinline__ void eval_otf3_fx(const arb_grid &g, const KParams &kp, const int64_t c[3],
                                              const double frac[3], double val[F], double grad[3]) {
   const int64_t nx = g.n[0], ny = g.n[1];
-  FxGrid3<F> src;
-  src.p = g.grid64 + ((c[2] * ny + c[1]) * nx + c[0]) * F;
-  src.sy = nx * F;
-  src.sz = nx * ny * F;
+  FxGrid3<F, STEP> src;
+  src.p = g.grid64 + ((c[2] * ny + c[1]) * nx + c[0]) * STEP + (STEP - F);
+  src.sy = nx * STEP;
+  src.sz = nx * ny * STEP;
   bool ok = src.template scale<false>();
   if (ok) {
     FxW wx, wy, wz;
@@ -624,7 +637,7 @@ __device__ __forceinline__ void eval_otf3_fx(const arb_grid &g, const KParams &k
     fx_finish3<F>(R, G, src.emax, kp.inv_h, val, grad);
     ok = src.fit();
   }
-  if (!ok) eval_otf3_slow<F>(g, kp, c, frac, val, grad);
+  if (!ok) eval_otf3_slow<F, STEP>(g, kp, c, frac, val, grad);
 }
 
 template <int F, bool MIXED>

@@ -457,13 +457,14 @@ struct FxMax {
 // largest corner, still 2^5 below the float64 rounding of those samples.
 constexpr int FX_HEAD = 3;
 
-template <int F>
+// STEP: doubles between points (F, or 4 for |B| of a 'both' grid alone).
+template <int F, int STEP = F>
 struct FxGrid3 {
   const double *p;  // block corner
   int64_t sy, sz;   // strides of y, z in doubles
   int emax[F];
   mutable uint32_t over[F];  // largest high word seen, per field
-  __device__ __forceinline__ const double *at(int i, int j, int k) const { return p + i * F + j * sy + k * sz; }
+  __device__ __forceinline__ const double *at(int i, int j, int k) const { return p + i * STEP + j * sy + k * sz; }
   __device__ __forceinline__ void point(int i, int j, int k, int h[F], int l[F]) const {
     uint32_t lo[F], hi[F];
     fx_read<F>(at(i, j, k), lo, hi);

@@ -188,7 +188,6 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
   const QRec64<3> *recs = reinterpret_cast<const QRec64<3> *>(w.rec);
   const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2];
   const int cls = bg.cls;
-  int turn = 0;
   for (int64_t b = blockIdx.x; b < bg.nbins; b += gridDim.x) {
     const uint32_t t0 = w.offs[b << cls], t1 = w.offs[(b + 1) << cls];
     if (t0 == t1) continue;
@@ -273,11 +272,7 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
       }
     }
     __syncthreads();
-    // warps start at another quarter of the records in each bin: the last,
-    // partial round of a bin would otherwise always fall to the same warps, and
-    // warp w of every CTA runs on scheduler w
-    const uint32_t first = t0 + ((threadIdx.x + 32u * (uint32_t)turn) % FX_THREADS);
-    ++turn;
+    const uint32_t first = t0 + threadIdx.x;
     // the next record is loaded while this one is evaluated
     QRec64<3> next;
     if (first < t1) next = recs[first];
@@ -385,7 +380,6 @@ __global__ void __launch_bounds__(FX_THREADS, F == 1 ? 3 : 2) eval_fx4_kernel(ar
   const QRec64<4> *recs = reinterpret_cast<const QRec64<4> *>(w.rec);
   const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2], nt = g.n[3];
   const int cls = bg.cls;
-  int turn = 0;
   for (int64_t b = blockIdx.x; b < bg.nbins; b += gridDim.x) {
     const uint32_t t0 = w.offs[b << cls], t1 = w.offs[(b + 1) << cls];
     if (t0 == t1) continue;
@@ -456,8 +450,7 @@ __global__ void __launch_bounds__(FX_THREADS, F == 1 ? 3 : 2) eval_fx4_kernel(ar
         }
     }
     __syncthreads();
-    const uint32_t first = t0 + ((threadIdx.x + 32u * (uint32_t)turn) % FX_THREADS);
-    ++turn;
+    const uint32_t first = t0 + threadIdx.x;
     for (uint32_t t = first; t < t1; t += FX_THREADS) {
       const QRec64<4> q = recs[t];
       int64_t c[4];

@@ -16,10 +16,44 @@
 
 namespace arb {
 
-// Acceleration at x; false when x is outside the interpolation volume.
-template <int F, bool MIXED>
-__device__ __forceinline__ bool rk4_accel(const arb_grid &g, const KParams &kp, const double x[3], double coef,
-                                          const double grav[3], double a[3]) {
+// |B| of a mixed 'both' grid as (hi, lo) pairs: the only field an integration
+// reads, 8 bytes a point where the grid's rows take 16 and 4.
+__global__ void __launch_bounds__(256) norm_pairs_kernel(const float *g32, int64_t npts, float2 *pairs) {
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (p < npts) pairs[p] = make_float2(__ldg(g32 + 4 * p + 3), __ldg(g32 + 4 * npts + p));
+}
+
+// Z-order key of each position over the interpolation box (10 bits per axis):
+// particles of one warp then gather neighbouring grid points.  Non-finite rows
+// sort last.  float32 is enough: the key orders the work, not the result.
+__device__ __forceinline__ uint32_t spread10(uint32_t v) {
+  v = (v | v << 16) & 0x030000ffu;
+  v = (v | v << 8) & 0x0300f00fu;
+  v = (v | v << 4) & 0x030c30c3u;
+  return (v | v << 2) & 0x09249249u;
+}
+__global__ void __launch_bounds__(256) zorder_kernel(const double *state, int64_t n, double l0, double l1, double l2,
+                                                     float s0, float s1, float s2, int32_t *keys) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double lo[3] = {l0, l1, l2};
+  const float sc[3] = {s0, s1, s2};
+  uint32_t key = 0;
+  bool finite = true;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float d = (float)(state[i * 6 + a] - lo[a]) * sc[a];
+    finite &= fabsf(d) < 1e30f;
+    key |= spread10((uint32_t)fminf(fmaxf(d, 0.f), 1023.f)) << a;
+  }
+  keys[i] = finite ? (int32_t)key : 1 << 30;
+}
+
+// Acceleration at x; false when x is outside the interpolation volume.  Only
+// the last field (the scalar, or |B|) and its gradient are evaluated.
+template <int F, bool MIXED, bool PAIRS>
+__device__ __forceinline__ bool rk4_accel(const arb_grid &g, const KParams &kp, const float2 *pairs, const double x[3],
+                                          double coef, const double grav[3], double a[3]) {
   using T = typename std::conditional<MIXED, float, double>::type;
   T fr[3];
   CoordStep s;
@@ -31,18 +65,36 @@ __device__ __forceinline__ bool rk4_accel(const arb_grid &g, const KParams &kp, 
   int64_t c[3];
   cell_from_step<3>(s, g, c);
   double val[F], grad[3] = {0.0, 0.0, 0.0};
-  eval_otf3<F, MIXED>(g, kp, c, fr, val, grad);
+  if constexpr (MIXED && PAIRS) {
+    NormBlock3 blk;
+    blk.v = pairs;
+    blk.sy = g.n[0];
+    blk.sz = g.n[0] * g.n[1];
+    blk.base = (c[2] * g.n[1] + c[1]) * g.n[0] + c[0];
+    eval_otf3_both_block(blk, kp, fr, val, grad);
+  } else if constexpr (MIXED) {
+    eval_otf3<F, MIXED>(g, kp, c, fr, val, grad);
+  } else {
+    eval_otf3_fx<1, F>(g, kp, c, fr, val, grad);
+  }
 #pragma unroll
   for (int a_ = 0; a_ < 3; ++a_) a[a_] = coef * grad[a_] + grav[a_];
   return true;
 }
 
-template <int F, bool MIXED>
-__global__ void __launch_bounds__(128, MIXED ? 1 : 3) rk4_kernel(arb_grid g, KParams kp, double *state, int64_t n, double dt,
+// Bound by L1 gathers and latency: |B| pairs take 8 bytes a point where the
+// 'both' grid takes 20, and 16 warps per SM (128 registers, a few spills) hide more
+// than 8 (2e5 particles x 25 steps on 128^3 'both', whole call: 3.87 ms; keys in
+// one kernel and no state copies, with pairs, 1.95; 16 warps 1.63).  float64: 13.7 ->
+// 3.7 ms with |B| alone in fixed point.
+template <int F, bool MIXED, bool PAIRS>
+__global__ void __launch_bounds__(128, MIXED ? 4 : 3) rk4_kernel(arb_grid g, KParams kp, const float2 *pairs,
+                                                                  const int64_t *order, double *state, int64_t n, double dt,
                                                   int64_t nsteps, double coef, double g0, double g1, double g2,
                                                   double *path, int64_t rec_every, unsigned long long *lost) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int64_t i = order ? order[t] : t;  // the particle
   double *st = state + i * 6;
   double x[3] = {st[0], st[1], st[2]}, v[3] = {st[3], st[4], st[5]};
   const double grav[3] = {g0, g1, g2};
@@ -69,7 +121,7 @@ __global__ void __launch_bounds__(128, MIXED ? 1 : 3) rk4_kernel(arb_grid g, KPa
         else
           xs[a] = x[a] + dt * (v[a] + h2 * k2v[a]);
       }
-      alive = rk4_accel<F, MIXED>(g, kp, xs, coef, grav, k);
+      alive = rk4_accel<F, MIXED, PAIRS>(g, kp, pairs, xs, coef, grav, k);
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         if (stg == 0)
@@ -118,28 +170,57 @@ __global__ void __launch_bounds__(128, MIXED ? 1 : 3) rk4_kernel(arb_grid g, KPa
 
 using namespace arb;
 
-extern "C" int arb_rk4_trajectories(const arb_grid *g, int32_t precision, double *state, int64_t n, double dt,
-                                    int64_t nsteps, double coef, const double *gravity, double *path,
-                                    int64_t record_every, unsigned long long *lost, arb_stream_t stream) {
+extern "C" int arb_rk4_trajectories_ordered(const arb_grid *g, int32_t precision, const float *pairs,
+                                            const int64_t *order, double *state, int64_t n, double dt,
+                                            int64_t nsteps, double coef, const double *gravity, double *path,
+                                            int64_t record_every, unsigned long long *lost, arb_stream_t stream) {
   if (!g || !state || !lost || n < 0 || nsteps < 0 || g->dim != 3) return ARB_ERR_INVALID;
   if (g->nfield == 3) return ARB_ERR_UNSUPPORTED;  // vector mode carries no gradient
   if (path && record_every <= 0) return ARB_ERR_INVALID;
   const bool mixed = precision == ARB_PREC_MIXED;
   if (mixed ? !g->grid32 : !g->grid64) return ARB_ERR_INVALID;
+  if (pairs && (!mixed || g->nfield != 4)) return ARB_ERR_INVALID;
   if (n == 0 || nsteps == 0) return ARB_OK;
   const double gr[3] = {gravity ? gravity[0] : 0.0, gravity ? gravity[1] : 0.0, gravity ? gravity[2] : 0.0};
   const KParams kp = make_kparams(g);
   cudaStream_t s = (cudaStream_t)stream;
   const int T = 128;
   const unsigned B = (unsigned)((n + T - 1) / T);
-#define RK(FF, MX)                                                                                        \
-  rk4_kernel<FF, MX><<<B, T, 0, s>>>(*g, kp, state, n, dt, nsteps, coef, gr[0], gr[1], gr[2], path, \
-                                     record_every, lost)
+#define RK(FF, MX, PR)                                                                                          \
+  rk4_kernel<FF, MX, PR><<<B, T, 0, s>>>(*g, kp, (const float2 *)pairs, order, state, n, dt, nsteps, coef, gr[0], \
+                                         gr[1], gr[2], path, record_every, lost)
   if (g->nfield == 1) {
-    if (mixed) RK(1, true); else RK(1, false);
+    if (mixed) RK(1, true, false); else RK(1, false, false);
+  } else if (mixed) {
+    if (pairs) RK(4, true, true); else RK(4, true, false);
   } else {
-    if (mixed) RK(4, true); else RK(4, false);
+    RK(4, false, false);
   }
 #undef RK
+  return launch_status();
+}
+
+extern "C" int arb_rk4_trajectories(const arb_grid *g, int32_t precision, double *state, int64_t n, double dt,
+                                    int64_t nsteps, double coef, const double *gravity, double *path,
+                                    int64_t record_every, unsigned long long *lost, arb_stream_t stream) {
+  return arb_rk4_trajectories_ordered(g, precision, nullptr, nullptr, state, n, dt, nsteps, coef, gravity, path,
+                                      record_every, lost, stream);
+}
+
+extern "C" int arb_norm_pairs(const arb_grid *g, float *pairs, arb_stream_t stream) {
+  if (!g || !g->grid32 || !pairs || g->nfield != 4 || g->dim != 3) return ARB_ERR_INVALID;
+  const int64_t npts = g->n[0] * g->n[1] * g->n[2];
+  norm_pairs_kernel<<<(unsigned)((npts + 255) / 256), 256, 0, (cudaStream_t)stream>>>(g->grid32, npts,
+                                                                                     (float2 *)pairs);
+  return launch_status();
+}
+
+extern "C" int arb_zorder_keys(const arb_grid *g, const double *state, int64_t n, int32_t *keys, arb_stream_t stream) {
+  if (!g || g->dim != 3 || n < 0 || (n > 0 && (!state || !keys))) return ARB_ERR_INVALID;
+  if (n == 0) return ARB_OK;
+  float sc[3];
+  for (int a = 0; a < 3; ++a) sc[a] = (float)(1023.0 / (g->hi[a] - g->lo[a]));
+  zorder_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(state, n, g->lo[0], g->lo[1], g->lo[2],
+                                                                              sc[0], sc[1], sc[2], keys);
   return launch_status();
 }

@@ -335,6 +335,19 @@ int arb_rk4_trajectories(const arb_grid *g, int32_t precision, double *state, in
                          int64_t nsteps, double coef, const double *gravity, double *path,
                          int64_t record_every, unsigned long long *lost, arb_stream_t stream);
 
+/* The same with two optional inputs that change no result: order, a
+ * permutation of the n particles in which threads take them (state and path
+ * stay in the caller's order; Z-order makes neighbouring threads gather
+ * neighbouring points), and pairs, |B| of a mixed 'both' grid as [npts] (hi, lo)
+ * floats written by arb_norm_pairs.  arb_zorder_keys writes one sort key per
+ * particle (30 bits; 1 << 30 for a non-finite position). */
+int arb_rk4_trajectories_ordered(const arb_grid *g, int32_t precision, const float *pairs, const int64_t *order,
+                                 double *state, int64_t n, double dt, int64_t nsteps, double coef,
+                                 const double *gravity, double *path, int64_t record_every,
+                                 unsigned long long *lost, arb_stream_t stream);
+int arb_norm_pairs(const arb_grid *g, float *pairs, arb_stream_t stream);
+int arb_zorder_keys(const arb_grid *g, const double *state, int64_t n, int32_t *keys, arb_stream_t stream);
+
 /* ---- field files: np.genfromtxt(path, delimiter=',') on the device
  *      (examples/3D_ARBInterpExample.py:14,37 and
  *      examples/4D_ARBInterpExample.py:14,38 load the N x 4..7 field tables
