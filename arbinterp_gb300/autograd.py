@@ -10,7 +10,7 @@ order: z-major, x fastest) and the query coordinates.  Forward runs the
 query kernels of ``libarbinterp.so``; backward runs ``arb_adjoint`` (atomic
 scatter of dL/dvalue and dL/dgrad through the Catmull-Rom weights, and
 dL/dq from the interpolant's gradient and Hessian), or in mixed precision
-with at least as many query rows as cells on ``arb_adjoint_binned`` (the
+with enough query rows per cell on ``arb_adjoint_binned`` (the
 same with the queries grouped by bin and the scatter accumulated per bin in
 shared memory).  A row whose upstream dL/dvalue is NaN scatters nothing and gets a
 NaN query gradient.
@@ -72,10 +72,11 @@ class TricubicFunction(torch.autograd.Function):
                 None if qg is None else qg.data_ptr())
         binned = ctx.field.binned_adjoint
         if binned is None:
-            # grouping pays once a bin holds several hundred queries (the
-            # binning passes, each bin's tile and one flush of its 1331
-            # points): at least as many queries as cells
-            binned = n >= max(interp.sort_threshold, interp.nc)
+            # grouping costs the binning passes, each bin's tile and one flush
+            # of its 1331 points: it pays from a sixth of the cells (86 queries
+            # a bin) on large sets (128^3: 5e5 queries 136 against 185 us, 2.5e5
+            # 108 against 99), on smaller ones from one query per cell
+            binned = n >= max(interp.sort_threshold, min(interp.nc, max(interp.nc // 6, 1 << 17)))
         if mixed and binned:
             # grouped by bin: dL/df accumulated per bin in shared memory
             need = int(L.arb_adjoint_work_bytes(interp._g, n))

@@ -180,16 +180,17 @@ __device__ __forceinline__ uint32_t fx_bits_at(const uint32_t *w, int o) {
 template <int F>
 __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(arb_grid g, KParams kp, BinGeom bg,
                                                                               int64_t nq, arb_query_out o,
-                                                                              SortedWork w) {
+                                                                              SortedWork w, uint32_t share) {
   extern __shared__ __align__(16) unsigned char fx_smem[];
   FxTile3<F> &tile = *reinterpret_cast<FxTile3<F> *>(fx_smem);
   __shared__ FxTileMax<F> smax;
   __shared__ uint32_t large_bits[F][(TILE_PTS + FX_THREADS) / 32 + 1];
   const QRec64<3> *recs = reinterpret_cast<const QRec64<3> *>(w.rec);
   const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2];
-  const int cls = bg.cls;
-  for (int64_t b = blockIdx.x; b < bg.nbins; b += gridDim.x) {
-    const uint32_t t0 = w.offs[b << cls], t1 = w.offs[(b + 1) << cls];
+  const BinItems items(w, bg, share);
+  for (int64_t it = blockIdx.x; it < items.n; it += gridDim.x) {
+    uint32_t t0, t1;
+    const int64_t b = items.get(it, t0, t1);
     if (t0 == t1) continue;
     const int64_t r = b / bg.nb[0];
     const int og[3] = {(int)((b % bg.nb[0]) * BIN_EDGE), (int)((r % bg.nb[1]) * BIN_EDGE),
@@ -372,16 +373,17 @@ struct FxRawSrc4 {
 
 template <int F>
 __global__ void __launch_bounds__(FX_THREADS, F == 1 ? 3 : 2) eval_fx4_kernel(arb_grid g, KParams kp, BinGeom bg, int64_t nq,
-                                                                 arb_query_out o, SortedWork w) {
+                                                                 arb_query_out o, SortedWork w, uint32_t share) {
   extern __shared__ __align__(16) unsigned char fx_smem[];
   FxTile4<F> &tile = *reinterpret_cast<FxTile4<F> *>(fx_smem);
   __shared__ FxTileMax<F> smax;
   __shared__ uint32_t large_bits[F][(TILE4_PTS + 31) / 32 + 1];
   const QRec64<4> *recs = reinterpret_cast<const QRec64<4> *>(w.rec);
   const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2], nt = g.n[3];
-  const int cls = bg.cls;
-  for (int64_t b = blockIdx.x; b < bg.nbins; b += gridDim.x) {
-    const uint32_t t0 = w.offs[b << cls], t1 = w.offs[(b + 1) << cls];
+  const BinItems items(w, bg, share);
+  for (int64_t it = blockIdx.x; it < items.n; it += gridDim.x) {
+    uint32_t t0, t1;
+    const int64_t b = items.get(it, t0, t1);
     if (t0 == t1) continue;
     int64_t og[4];
     bin_origin4(b, bg, og);
@@ -535,16 +537,18 @@ template <int DIM, int F>
 static bool launch_eval_fx_f(const arb_grid *g, const KParams &kp, const BinGeom &bg, int64_t nq,
                              const arb_query_out *out, const SortedWork &w, cudaStream_t s) {
   static int per_sm[MAX_DEVICES] = {};
+  const uint32_t share = split_share(bg, nq);
+  const int64_t items = bg.nbins + nq / share;  // at most
   if constexpr (DIM == 3) {
     int64_t grid = fx_grid(eval_fx3_kernel<F>, sizeof(FxTile3<F>), per_sm);
     if (!grid) return false;
-    if (grid > bg.nbins) grid = bg.nbins;
-    eval_fx3_kernel<F><<<(unsigned)grid, FX_THREADS, sizeof(FxTile3<F>), s>>>(*g, kp, bg, nq, *out, w);
+    if (grid > items) grid = items;
+    eval_fx3_kernel<F><<<(unsigned)grid, FX_THREADS, sizeof(FxTile3<F>), s>>>(*g, kp, bg, nq, *out, w, share);
   } else {
     int64_t grid = fx_grid(eval_fx4_kernel<F>, sizeof(FxTile4<F>), per_sm);
     if (!grid) return false;
-    if (grid > bg.nbins) grid = bg.nbins;
-    eval_fx4_kernel<F><<<(unsigned)grid, FX_THREADS, sizeof(FxTile4<F>), s>>>(*g, kp, bg, nq, *out, w);
+    if (grid > items) grid = items;
+    eval_fx4_kernel<F><<<(unsigned)grid, FX_THREADS, sizeof(FxTile4<F>), s>>>(*g, kp, bg, nq, *out, w, share);
   }
   return true;
 }

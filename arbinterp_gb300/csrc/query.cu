@@ -21,7 +21,7 @@
 namespace arb {
 
 template <int F, bool MIXED>
-__global__ void __launch_bounds__(256, MIXED ? 1 : 2) otf3_kernel(arb_grid g, KParams kp, double *q, int64_t nq,
+__global__ void __launch_bounds__(256, MIXED && F != 1 ? 0 : 2) otf3_kernel(arb_grid g, KParams kp, double *q, int64_t nq,
                                                    int64_t qs, int wb, arb_query_out o,
                                                    int32_t *status) {
   using T = typename std::conditional<MIXED, float, double>::type;
@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256, MIXED ? 1 : 2) otf3_kernel(arb_grid g, KP
 }
 
 template <int F, bool MIXED>
-__global__ void __launch_bounds__(128, MIXED ? 1 : 3) otf4_kernel(arb_grid g, KParams kp, double *q, int64_t nq,
+__global__ void __launch_bounds__(128, MIXED ? 0 : 3) otf4_kernel(arb_grid g, KParams kp, double *q, int64_t nq,
                                                    int64_t qs, int wb, arb_query_out o,
                                                    int32_t *status) {
   using T = typename std::conditional<MIXED, float, double>::type;

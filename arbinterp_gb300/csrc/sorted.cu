@@ -468,8 +468,68 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const uint32_t
   }
 }
 
+// ---- shares of crowded bins ----------------------------------------------------
+// A staged kernel takes one bin per CTA.  Clouds crowd a few bins, and small
+// grids have fewer bins than the GPU has CTAs, so a bin of more than `share`
+// records is cut: its first share is the bin's own item, each further one an
+// item (bin, share number) in the list that split_kernel leaves in the
+// histogram (which placement has counted down to zero; word 0 is the list's
+// length).  split_share bounds the list by the room there.
+struct BinItem {
+  uint32_t bin, part;
+};
+
+// About four items for each of ~600 resident CTAs.  Where the bins alone make
+// two, only a bin of twice the mean is cut (its tile is staged again for every
+// share: cutting 1220-record bins at 512 cost 10 %).  At least 512, and nq / 6 a
+// bin at most, for the list's room.
+static inline uint32_t split_share(const BinGeom &bg, int64_t nq) {
+  int64_t s = nq / 2432;
+  if (bg.nbins >= 1216 && s < 2 * nq / bg.nbins) s = 2 * nq / bg.nbins;
+  if (s < nq / (6 * bg.nbins)) s = nq / (6 * bg.nbins);
+  return (uint32_t)(s + 1 > 512 ? s + 1 : 512);
+}
+
+__global__ void __launch_bounds__(256) split_kernel(const uint32_t *offs, BinGeom bg, uint32_t share, uint32_t *hist) {
+  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (b >= bg.nbins) return;
+  const uint32_t n = offs[(b + 1) << bg.cls] - offs[b << bg.cls];
+  if (n <= share) return;
+  const uint32_t more = (n - 1) / share, at = atomicAdd(hist, more);
+  for (uint32_t p = 0; p < more; ++p)
+    reinterpret_cast<uint2 *>(hist + 2)[at + p] = make_uint2((uint32_t)b, p + 1);
+}
+
+// The items of a staged kernel: the further shares first (each a full one or
+// the rest of a crowded bin), then every bin's own.
+struct BinItems {
+  const uint32_t *offs;
+  const uint2 *more;
+  int64_t nmore, n;
+  uint32_t share;
+  int cls;
+  __device__ __forceinline__ BinItems(const SortedWork &w, const BinGeom &bg, uint32_t share_)
+      : offs(w.offs), more(reinterpret_cast<const uint2 *>(w.hist + 2)), nmore(w.hist[0]), n(nmore + bg.nbins),
+        share(share_), cls(bg.cls) {}
+  // Bin of item i and its records [t0, t1); t0 == t1 past the end.
+  __device__ __forceinline__ int64_t get(int64_t i, uint32_t &t0, uint32_t &t1) const {
+    t0 = t1 = 0;
+    if (i >= n) return 0;
+    int64_t b = i - nmore;
+    uint32_t part = 0;
+    if (b < 0) {
+      const uint2 m = more[i];
+      b = m.x;
+      part = m.y;
+    }
+    t0 = offs[b << cls] + part * share;
+    t1 = min(offs[(b + 1) << cls], t0 + share);
+    return b;
+  }
+};
+
 template <int DIM, int F, bool MIXED, bool TABLE>
-__global__ void __launch_bounds__(DIM == 3 ? 256 : 128, MIXED ? 1 : (DIM == 3 ? 2 : 3)) eval_sorted_kernel(arb_grid g, KParams kp,
+__global__ void __launch_bounds__(DIM == 3 ? 256 : 128, MIXED ? 0 : (DIM == 3 ? 2 : 3)) eval_sorted_kernel(arb_grid g, KParams kp,
                                                                            int64_t nq, arb_query_out o,
                                                                            SortedWork w) {
   using T = typename std::conditional<MIXED, float, double>::type;
@@ -620,15 +680,11 @@ struct TileBlock3<3> {
 // of the bin, which placement wrote in the bin's bank schedule.
 template <int F>
 __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) eval_binc_kernel(arb_grid g, KParams kp, BinGeom bg,
-                                                                   int64_t nq, arb_query_out o, SortedWork w) {
+                                                                   int64_t nq, arb_query_out o, SortedWork w, uint32_t share) {
   extern __shared__ __align__(16) unsigned char binc_smem[];
   BinTile<F> *tiles = reinterpret_cast<BinTile<F> *>(binc_smem);
-  const int64_t nbins = bg.nbins;
   const QRec *recs = reinterpret_cast<const QRec *>(w.rec);
-  // bin b holds records [offs[16 b], offs[16 b + 16]) (its 16 class sub-bins)
-  const int cls = bg.cls;
-  auto begin = [&](int64_t bb) { return w.offs[bb << cls]; };
-  auto count = [&](int64_t bb) { return bb < nbins ? w.offs[(bb + 1) << cls] - begin(bb) : 0u; };
+  const BinItems items(w, bg, share);
   auto origin = [&](int64_t bb, int og[3]) {
     og[0] = (int)((bb % bg.nb[0]) * BIN_EDGE);
     const int64_t r = bb / bg.nb[0];
@@ -636,25 +692,20 @@ __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) e
     og[2] = (int)((r / bg.nb[1]) * BIN_EDGE);
   };
   int stage = 0;
-  int64_t b = blockIdx.x;
-  int og[3];
-  if (count(b) > 0) {
-    origin(b, og);
-    load_bin_tile<F>(g, og, tiles[0]);
-  }
+  int og[3], on[3];
+  uint32_t t0, t1, n0, n1;
+  int64_t b = items.get(blockIdx.x, t0, t1);
+  origin(b, og);
+  if (t1 > t0) load_bin_tile<F>(g, og, tiles[0]);
   cp_async_commit();
-  for (; b < nbins; b += gridDim.x) {
-    const int64_t bn = b + gridDim.x;
-    if (count(bn) > 0) {
-      origin(bn, og);
-      load_bin_tile<F>(g, og, tiles[stage ^ 1]);
-    }
+  for (int64_t it = blockIdx.x; it < items.n; it += gridDim.x) {
+    b = items.get(it + gridDim.x, n0, n1);
+    origin(b, on);
+    if (n1 > n0) load_bin_tile<F>(g, on, tiles[stage ^ 1]);
     cp_async_commit();
-    const uint32_t t0 = begin(b), t1 = t0 + count(b);
     cp_async_wait1();
     __syncthreads();
     if (t1 > t0) {
-      origin(b, og);
       // the next record is loaded while this one is evaluated
       QRec rnext;
       if (t0 + threadIdx.x < t1) rnext = recs[t0 + threadIdx.x];
@@ -683,8 +734,12 @@ __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) e
         write_vals<3, F>(o, r.row, val, grad);
       }
     }
-    __syncthreads();  // this stage is refilled two bins later
+    __syncthreads();  // this stage is refilled two items later
     stage ^= 1;
+    t0 = n0;
+    t1 = n1;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) og[a] = on[a];
   }
   // records that need no evaluation (out of volume, NaN, sentinel column)
   for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
@@ -717,9 +772,10 @@ static bool launch_eval_binc_f(const arb_grid *g, const KParams &kp, const BinGe
     per_sm[dev] = n;
   }
   int64_t grid = (int64_t)sm_count_sorted() * per_sm[dev];
-  if (grid > bg.nbins) grid = bg.nbins;
-  if (grid < 1) grid = 1;
-  eval_binc_kernel<F><<<(unsigned)grid, BINC_THREADS, smem, s>>>(*g, kp, bg, nq, *out, w);
+  const uint32_t share = split_share(bg, nq);
+  const int64_t items = bg.nbins + nq / share;  // at most
+  if (grid > items) grid = items;
+  eval_binc_kernel<F><<<(unsigned)grid, BINC_THREADS, smem, s>>>(*g, kp, bg, nq, *out, w, share);
   return true;
 }
 
@@ -796,31 +852,26 @@ __device__ __forceinline__ void load_bin_tile4(const arb_grid &g, const BinGeom 
 }
 
 __global__ void __launch_bounds__(BIN4_THREADS) eval_bin4_kernel(arb_grid g, KParams kp, BinGeom bg, int64_t nq,
-                                                                 arb_query_out o, SortedWork w) {
+                                                                 arb_query_out o, SortedWork w, uint32_t share) {
   extern __shared__ __align__(16) unsigned char bin4_smem[];
   BinTile4 *tiles = reinterpret_cast<BinTile4 *>(bin4_smem);
-  const int64_t nbins = bg.nbins;
   const QRec *recs = reinterpret_cast<const QRec *>(w.rec);
+  const BinItems items(w, bg, share);
   int stage = 0;
-  int64_t b = blockIdx.x;
-  // bin b holds records [offs[b << cls], offs[(b + 1) << cls]) (its class
-  // sub-bins, in the bin's bank schedule); bins with no query need no copy
-  const int cls = bg.cls;
-  auto bin_begin = [&](int64_t bb) { return (int64_t)w.offs[bb << cls]; };
-  auto count = [&](int64_t bb) { return bb < nbins ? (int64_t)w.offs[(bb + 1) << cls] - bin_begin(bb) : 0; };
-  if (count(b) > 0) load_bin_tile4(g, bg, b, tiles[0]);
+  uint32_t t0, t1, n0, n1;
+  int64_t b = items.get(blockIdx.x, t0, t1);
+  if (t1 > t0) load_bin_tile4(g, bg, b, tiles[0]);
   cp_async_commit();
-  for (; b < nbins; b += gridDim.x) {
-    const int64_t bn = b + gridDim.x;
-    if (count(bn) > 0) load_bin_tile4(g, bg, bn, tiles[stage ^ 1]);
+  for (int64_t it = blockIdx.x; it < items.n; it += gridDim.x) {
+    const int64_t bn = items.get(it + gridDim.x, n0, n1);
+    if (n1 > n0) load_bin_tile4(g, bg, bn, tiles[stage ^ 1]);
     cp_async_commit();
-    const int64_t t0 = bin_begin(b), t1 = w.offs[(b + 1) << cls];
     cp_async_wait1();
     __syncthreads();
     if (t1 > t0) {
       int64_t og[4];
       bin_origin4(b, bg, og);
-      for (int64_t t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
+      for (uint32_t t = t0 + threadIdx.x; t < t1; t += BIN4_THREADS) {
         const QRec r = recs[t];
         int64_t c[4];
         unpack_cell<4>(r.cell, c);
@@ -835,8 +886,11 @@ __global__ void __launch_bounds__(BIN4_THREADS) eval_bin4_kernel(arb_grid g, KPa
         write_vals<4, 1>(o, r.row, val, grad);
       }
     }
-    __syncthreads();  // this stage is refilled two bins later
+    __syncthreads();  // this stage is refilled two items later
     stage ^= 1;
+    b = bn;
+    t0 = n0;
+    t1 = n1;
   }
   // records that need no evaluation (out of volume, NaN, sentinel column)
   for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
@@ -866,9 +920,10 @@ static bool launch_eval_bin4(const arb_grid *g, const KParams &kp, const BinGeom
     per_sm[dev] = n;
   }
   int64_t grid = (int64_t)sm_count_sorted() * per_sm[dev];
-  if (grid > bg.nbins) grid = bg.nbins;
-  if (grid < 1) grid = 1;
-  eval_bin4_kernel<<<(unsigned)grid, BIN4_THREADS, smem, s>>>(*g, kp, bg, nq, *out, w);
+  const uint32_t share = split_share(bg, nq);
+  const int64_t items = bg.nbins + nq / share;  // at most
+  if (grid > items) grid = items;
+  eval_bin4_kernel<<<(unsigned)grid, BIN4_THREADS, smem, s>>>(*g, kp, bg, nq, *out, w, share);
   return true;
 }
 
@@ -888,6 +943,7 @@ static void launch_bin(const arb_grid *g, const KParams &kp, const BinGeom &bg, 
   scan_part_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(w.hist, nh, w.part);
   scan_apply_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(w.hist, nh, w.part, w.offs, w.hdr, bg.nbins);
   bin_place_kernel<DIM, !MIXED, T><<<B, TB, 0, s>>>(*g, kp, bg, q, nq, qs, w);
+  if (bg.cls) split_kernel<<<(unsigned)((bg.nbins + 255) / 256), 256, 0, s>>>(w.offs, bg, split_share(bg, nq), w.hist);
 }
 
 // Table evaluation, 8 lanes per query.  A cell's block is F fields x R rows
@@ -1018,24 +1074,28 @@ static void launch_eval(const arb_grid *g, const KParams &kp, int64_t nq, const 
 // The backward of rQuery2 (ARBInterp.py:399-454), as arb_adjoint computes it
 // per query, but grouped by the 8^3-cell bins of the query pass: the bin's
 // (hi, lo) tile is staged as for the forward (the dL/dq terms read the
-// interpolant's gradient and Hessian from it), and dL/df is accumulated in a
-// shared-memory tile of the bin's 11^3 points with shared atomics, then
-// added to the grid gradient once per point and bin.  A query scatters 64
-// values, so with ~250 queries per bin (1e6 queries on 128^3) the global
-// atomics fall from 64 per query to 1331 per bin.
+// interpolant's gradient and Hessian from it), and dL/df is accumulated in
+// shared-memory tiles of the bin's 11^3 points, then added to the grid
+// gradient once per point and bin.
+//
+// Every warp has a tile of its own and adds with plain loads and stores.  At
+// one point (i, j, k) of their blocks two lanes meet in an address only if
+// their queries lie in the same cell: such lanes take turns (two rounds as a
+// rule), and the steps of a warp are ordered.  Float atomics in shared memory
+// are compare-and-swap loops and were the kernel's first stall (1e6 queries on
+// 128^3: 202 us).
 constexpr int ADJ_THREADS = 128;
+constexpr int ADJ_WARPS = ADJ_THREADS / 32;
 
 __global__ void __launch_bounds__(ADJ_THREADS) adjoint_bin_kernel(arb_grid g, KParams kp, BinGeom bg, int64_t nq,
                                                                   const double *dval, const double *dgrad,
-                                                                  float *grid_grad, double *q_grad, SortedWork w) {
+                                                                  float *grid_grad, double *q_grad, SortedWork w, uint32_t share) {
   extern __shared__ __align__(16) unsigned char adj_smem[];
   BinTile<1> *tiles = reinterpret_cast<BinTile<1> *>(adj_smem);
-  float *gt = reinterpret_cast<float *>(adj_smem + 2 * sizeof(BinTile<1>));  // dL/df of the bin's points
-  const int64_t nbins = bg.nbins;
+  float *gts = reinterpret_cast<float *>(adj_smem + 2 * sizeof(BinTile<1>));  // dL/df of the bin's points, per warp
+  volatile float *gt = gts + threadIdx.x / 32 * TILE_PTS;
   const QRec *recs = reinterpret_cast<const QRec *>(w.rec);
-  const int cls = bg.cls;
-  auto begin = [&](int64_t bb) { return w.offs[bb << cls]; };
-  auto count = [&](int64_t bb) { return bb < nbins ? w.offs[(bb + 1) << cls] - begin(bb) : 0u; };
+  const BinItems items(w, bg, share);
   auto origin = [&](int64_t bb, int og[3]) {
     og[0] = (int)((bb % bg.nb[0]) * BIN_EDGE);
     const int64_t r = bb / bg.nb[0];
@@ -1044,70 +1104,87 @@ __global__ void __launch_bounds__(ADJ_THREADS) adjoint_bin_kernel(arb_grid g, KP
   };
   const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2];
   const float ih[3] = {kp.inv_hf[0], kp.inv_hf[1], kp.inv_hf[2]};
-  for (int e = threadIdx.x; e < TILE_PTS; e += blockDim.x) gt[e] = 0.f;
+  for (int e = threadIdx.x; e < ADJ_WARPS * TILE_PTS; e += ADJ_THREADS) gts[e] = 0.f;
   int stage = 0;
-  int64_t b = blockIdx.x;
-  int og[3];
-  if (count(b) > 0) {
-    origin(b, og);
-    load_bin_tile<1>(g, og, tiles[0]);
-  }
+  int og[3], onx[3];
+  uint32_t t0, t1, n0, n1;
+  int64_t b = items.get(blockIdx.x, t0, t1);
+  origin(b, og);
+  if (t1 > t0) load_bin_tile<1>(g, og, tiles[0]);
   cp_async_commit();
-  for (; b < nbins; b += gridDim.x) {
-    const int64_t bn = b + gridDim.x;
-    if (count(bn) > 0) {
-      origin(bn, og);
-      load_bin_tile<1>(g, og, tiles[stage ^ 1]);
-    }
+  for (int64_t it = blockIdx.x; it < items.n; it += gridDim.x) {
+    b = items.get(it + gridDim.x, n0, n1);
+    origin(b, onx);
+    if (n1 > n0) load_bin_tile<1>(g, onx, tiles[stage ^ 1]);
     cp_async_commit();
-    const uint32_t t0 = begin(b), t1 = t0 + count(b);
     cp_async_wait1();
     __syncthreads();
     if (t1 > t0) {
-      origin(b, og);
       const float2 *tv = tiles[stage].v;
-      for (uint32_t t = t0 + threadIdx.x; t < t1; t += ADJ_THREADS) {
-        const QRec r = recs[t];
+      for (uint32_t tw = t0 + threadIdx.x / 32 * 32; tw < t1; tw += ADJ_THREADS) {  // warps stay whole
+        const uint32_t t = tw + (threadIdx.x & 31);
+        bool on = t < t1;
+        const QRec r = recs[on ? t : t0];
         const int64_t row = r.row;
-        const float dv = dval ? (float)dval[row] : 0.f;
+        const float dv = on && dval ? (float)dval[row] : 0.f;
         float dg[3] = {0.f, 0.f, 0.f};
-        if (dgrad) {
+        if (on && dgrad) {
           dg[0] = (float)dgrad[row * 3];
           dg[1] = (float)dgrad[row * 3 + 1];
           dg[2] = (float)dgrad[row * 3 + 2];
         }
-        if (dv != dv) {  // a NaN upstream: no scatter, a NaN query gradient
+        if (on && dv != dv) {  // a NaN upstream: no scatter, a NaN query gradient
           if (q_grad) q_grad[row * 3] = q_grad[row * 3 + 1] = q_grad[row * 3 + 2] = qnan();
-          continue;
+          on = false;
         }
         int64_t c[3];
         unpack_cell<3>(r.cell, c);
         const int base = (((int)c[2] - og[2]) * TILE_EDGE + ((int)c[1] - og[1])) * TILE_EDGE + ((int)c[0] - og[0]);
-        float wgt[3][4], d1[3][4], d2[3][4];
+        float wgt[3][4], d1[3][4];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           cr_weights<float>(r.f[a], wgt[a]);
           cr_dweights<float>(r.f[a], d1[a]);
-          cr_d2weights<float>(r.f[a], d2[a]);
         }
         const float gx = dg[0] * ih[0], gy = dg[1] * ih[1], gz = dg[2] * ih[2];
-        float G[3] = {0.f, 0.f, 0.f}, H[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // H: xx yy zz xy xz yz
+        // turns of the lanes of one cell (lanes without a scatter: none)
+        const unsigned peers = __match_any_sync(0xffffffffu, on ? base : -1 - (int)(threadIdx.x & 31));
+        const int turn = on ? __popc(peers & ((1u << (threadIdx.x & 31)) - 1u)) : -1;
+        const int turns = __reduce_max_sync(0xffffffffu, turn) + 1;
+        for (int n = 0; n < turns; ++n) {
+          const bool mine = turn == n;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+          for (int k = 0; k < 4; ++k) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int p = base + (k * TILE_EDGE + j) * TILE_EDGE;
-            const float yz = wgt[1][j] * wgt[2][k];
-            float f[4];
+            for (int j = 0; j < 4; ++j) {
+              const float yz = wgt[1][j] * wgt[2][k];
+              const float c0 = dv * yz + gy * (d1[1][j] * wgt[2][k]) + gz * (wgt[1][j] * d1[2][k]), c1 = gx * yz;
 #pragma unroll
-            for (int ii = 0; ii < 4; ++ii) {
-              const float2 hl = tv[p + ii];
-              f[ii] = hl.x + hl.y;
-              const float cval = dv * wgt[0][ii] * yz + gx * d1[0][ii] * yz + gy * wgt[0][ii] * d1[1][j] * wgt[2][k] +
-                                 gz * wgt[0][ii] * wgt[1][j] * d1[2][k];
-              if (cval != 0.f) atomicAdd(gt + p + ii, cval);
+              for (int ii = 0; ii < 4; ++ii) {
+                const int p = base + (k * TILE_EDGE + j) * TILE_EDGE + ii;
+                if (mine) gt[p] = gt[p] + (wgt[0][ii] * c0 + d1[0][ii] * c1);
+                __syncwarp();
+              }
             }
-            if (q_grad) {
+          }
+        }
+        if (q_grad && on) {
+          float d2[3][4];
+#pragma unroll
+          for (int a = 0; a < 3; ++a) cr_d2weights<float>(r.f[a], d2[a]);
+          float G[3] = {0.f, 0.f, 0.f}, H[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // H: xx yy zz xy xz yz
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int p = base + (k * TILE_EDGE + j) * TILE_EDGE;
+              const float yz = wgt[1][j] * wgt[2][k];
+              float f[4];
+#pragma unroll
+              for (int ii = 0; ii < 4; ++ii) {
+                const float2 hl = tv[p + ii];
+                f[ii] = hl.x + hl.y;
+              }
               const float a0 = wgt[0][0] * f[0] + wgt[0][1] * f[1] + wgt[0][2] * f[2] + wgt[0][3] * f[3];
               const float a1 = d1[0][0] * f[0] + d1[0][1] * f[1] + d1[0][2] * f[2] + d1[0][3] * f[3];
               const float a2 = d2[0][0] * f[0] + d2[0][1] * f[1] + d2[0][2] * f[2] + d2[0][3] * f[3];
@@ -1122,8 +1199,6 @@ __global__ void __launch_bounds__(ADJ_THREADS) adjoint_bin_kernel(arb_grid g, KP
               H[5] += a0 * d1[1][j] * d1[2][k];
             }
           }
-        }
-        if (q_grad) {
           const float Hm[3][3] = {{H[0], H[3], H[4]}, {H[3], H[1], H[5]}, {H[4], H[5], H[2]}};
 #pragma unroll
           for (int a = 0; a < 3; ++a) {
@@ -1135,19 +1210,27 @@ __global__ void __launch_bounds__(ADJ_THREADS) adjoint_bin_kernel(arb_grid g, KP
         }
       }
     }
-    __syncthreads();  // the bin's scatter is complete; this stage is refilled two bins later
+    __syncthreads();  // the bin's scatter is complete; this stage is refilled two items later
     if (t1 > t0) {
       // one global atomic per touched point of the bin (each thread clears what it flushes)
-      for (int e = threadIdx.x; e < TILE_PTS; e += blockDim.x) {
-        const float v = gt[e];
+      for (int e = threadIdx.x; e < TILE_PTS; e += ADJ_THREADS) {
+        float v = 0.f;
+#pragma unroll
+        for (int m = 0; m < ADJ_WARPS; ++m) {
+          v += gts[m * TILE_PTS + e];
+          gts[m * TILE_PTS + e] = 0.f;
+        }
         if (v == 0.f) continue;
-        gt[e] = 0.f;
         const int lx = e % TILE_EDGE, rr = e / TILE_EDGE;
         const int64_t x = og[0] + lx, y = og[1] + rr % TILE_EDGE, z = og[2] + rr / TILE_EDGE;
         if (x < nx && y < ny && z < nz) atomicAdd(grid_grad + (z * ny + y) * nx + x, v);
       }
     }
     stage ^= 1;
+    t0 = n0;
+    t1 = n1;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) og[a] = onx[a];
   }
   // rows outside the volume, NaN rows and the sentinel column: no gradient
   if (q_grad)
@@ -1385,21 +1468,24 @@ extern "C" int arb_adjoint_binned(const arb_grid *g, int32_t precision, const do
   if (cudaMemsetAsync(w.hist, 0, sizeof(uint32_t) * (bg.nsub + 1), s) != cudaSuccess) return ARB_ERR_CUDA;
   const KParams kp = make_kparams(&gb);
   launch_bin<3, true>(&gb, kp, bg, const_cast<double *>(q), nq, q_stride, 0, &out, status, w, s);
-  const size_t smem = 2 * sizeof(BinTile<1>) + sizeof(float) * TILE_PTS;
+  const size_t smem = 2 * sizeof(BinTile<1>) + sizeof(float) * TILE_PTS * ADJ_WARPS;
   static int per_sm[MAX_DEVICES] = {};
   const int dev = current_device();
   if (dev < 0) return ARB_ERR_CUDA;
   if (!per_sm[dev]) {
     int n = 0;
+    if (cudaFuncSetAttribute(adjoint_bin_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return ARB_ERR_CUDA;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjoint_bin_kernel, ADJ_THREADS, smem) != cudaSuccess ||
         n < 1)
       return ARB_ERR_CUDA;
     per_sm[dev] = n;
   }
   int64_t grid = (int64_t)sm_count_sorted() * per_sm[dev];
-  if (grid > bg.nbins) grid = bg.nbins;
-  if (grid < 1) grid = 1;
+  const uint32_t share = split_share(bg, nq);
+  const int64_t items = bg.nbins + nq / share;  // at most
+  if (grid > items) grid = items;
   adjoint_bin_kernel<<<(unsigned)grid, ADJ_THREADS, smem, s>>>(gb, kp, bg, nq, dval, dgrad, (float *)grid_grad,
-                                                               q_grad, w);
+                                                               q_grad, w, share);
   return launch_status();
 }
