@@ -254,6 +254,66 @@ __device__ __forceinline__ bool norm_f32pair(double bx, double by, double bz, fl
   return true;
 }
 
+// Correctly rounded float64 square root on the integer and float32 pipes (the
+// float64 pipe, 2 lanes per SM and clock, made the fill of a 'both' grid wait:
+// ~11 operations a root).  With s = m 2^E, the root's significand is Q =
+// floor(sqrt(m 2^t)) in [2^52, 2^53): a float32 estimate (23 bits), one step on
+// the residual's upper bits and one on the exact residual modulo 2^64 bring Q
+// within one; Q^2 <= S < (Q + 1)^2 decides it, and S - Q^2 > Q the rounding (a
+// root is never halfway).
+__host__ __device__ __forceinline__ bool sqrt_bits(unsigned long long b, unsigned long long &root) {
+  const int e = (int)(b >> 52);
+  if (e < 64 || e > 2046) return false;  // zero, tiny, negative, infinity, NaN: the caller's
+  const unsigned long long m = (b & 0xfffffffffffffULL) | 0x10000000000000ULL;
+  const int t = 52 + ((e + 1) & 1);  // e - 1075 - t is even
+  const unsigned ab = (unsigned)(m >> 29) - 0x800000u + ((unsigned)(127 + t - 52) << 23);
+  float a, y;
+  unsigned k;
+#ifdef __CUDA_ARCH__
+  a = __uint_as_float(ab);
+  y = rsqrtf(a);
+#else
+  memcpy(&a, &ab, 4);
+  y = 1.f / sqrtf(a);
+#endif
+  float q = a * y;  // one Newton step: within a unit in the last place of 24 bits
+  q = fmaf(fmaf(-q, q, a), 0.5f * y, q);
+#ifdef __CUDA_ARCH__
+  k = __float_as_uint(q);
+#else
+  memcpy(&k, &q, 4);
+#endif
+  k = k >= 0x40000000u ? 0xffffffu : ((k & 0x7fffffu) | 0x800000u);
+  unsigned long long Q = (unsigned long long)k << 29;
+  // (S - Q^2) / 2^40, then its half over Q
+  const long long R = (long long)((m << (t - 40)) - (((unsigned long long)k * k) << 18));
+  Q += (long long)((int)((float)(int)(R >> 13) * y));  // |R| < 2^44
+  long long r = (long long)((m << t) - Q * Q);
+  const int d = (int)((float)(int)(r >> 32) * y * 0x1p-21f);
+  Q += (long long)d;
+  r = (long long)((m << t) - Q * Q);
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    if (r < 0) {
+      --Q;
+      r += (long long)(2 * Q + 1);
+    } else if (r > (long long)(2 * Q)) {
+      r -= (long long)(2 * Q + 1);
+      ++Q;
+    }
+  }
+  if (r > (long long)Q) ++Q;
+  root = ((unsigned long long)(unsigned)((e - 1075 - t) / 2 + 1074) << 52) + Q;  // Q carries its leading one
+  return true;
+}
+
+__device__ __noinline__ double sqrt_slow(double v) { return __dsqrt_rn(v); }
+__device__ __forceinline__ double sqrt_f64(double v) {
+  unsigned long long r;
+  if (sqrt_bits(opaque_u64((unsigned long long)__double_as_longlong(v)), r)) return __longlong_as_double((long long)r);
+  return sqrt_slow(v);
+}
+
 // Per-mode interpolated fields of one row written to grid slot `dest`:
 // grid64, grid32 (hi/lo split, layout of g32_load in arb_common.cuh) and the
 // raw value columns.  With grid32 (mixed precision) and float64 components
@@ -282,8 +342,8 @@ __device__ __forceinline__ void write_slot(const TF *row, int64_t dest, int64_t 
         nrm = grid64 ? f2d_exact(nhi) + f2d_exact(nlo) : 0.0;
         nsplit = true;
       } else if (sizeof(TF) == 8) {
-        nrm = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn((double)bx, (double)bx), __dmul_rn((double)by, (double)by)),
-                                   __dmul_rn((double)bz, (double)bz)));
+        nrm = sqrt_f64(__dadd_rn(__dadd_rn(__dmul_rn((double)bx, (double)bx), __dmul_rn((double)by, (double)by)),
+                                 __dmul_rn((double)bz, (double)bz)));
       } else {
         nrm = f2d_exact(__fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn((float)bx, (float)bx), __fmul_rn((float)by, (float)by)),
                                              __fmul_rn((float)bz, (float)bz))));
