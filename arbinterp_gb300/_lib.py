@@ -60,12 +60,15 @@ SIGNATURES = {
                                            _P, _P]),
     "arb_ingest_ordered_fill": (C.c_int, [_P, _I32, _I64, _I32, _I32, _I32, _I64, _P, _P, C.c_size_t, _P, _P,
                                           _P, _P, _P]),
+    "arb_ingest_ordered_start": (C.c_int, [_P, _I32, _I64, _I32, _I32, _I32, _I64, _P, _P, _P, C.c_size_t, _P, _P,
+                                           _P]),
     "arb_ingest_summary": (C.c_int, [_P, _I64, _P, _I32, _P, _P, _P]),
     "arb_fd_planes": (C.c_int, [C.POINTER(ArbGrid), _P, _P]),
     "arb_coef_solve": (C.c_int, [C.POINTER(ArbGrid), _I32, _I64, _I64, _P, _P, _P]),
     "arb_query_eval": (C.c_int, [C.POINTER(ArbGrid), _P, _I64, _I64, _I32, C.POINTER(ArbQueryOut), _P, _P]),
     "arb_query_eval_otf": (C.c_int, [C.POINTER(ArbGrid), _I32, _P, _I64, _I64, _I32,
                                      C.POINTER(ArbQueryOut), _P, _P]),
+    "arb_query_point": (C.c_int, [C.POINTER(ArbGrid), _I32, _I32, C.POINTER(C.c_double), _P, _P, _P]),
     "arb_query_sorted_work_bytes": (C.c_size_t, [C.POINTER(ArbGrid), _I32, _I64]),
     "arb_query_eval_sorted": (C.c_int, [C.POINTER(ArbGrid), _I32, _I32, _P, _I64, _I64, _I32,
                                         C.POINTER(ArbQueryOut), _P, C.c_size_t, _P, _P]),

@@ -99,13 +99,13 @@ __device__ __forceinline__ void write_vals(const arb_query_out &o, int64_t i, co
 // Returns true when the row still needs evaluating.
 // EXACT (float64 path): the IEEE quotient, frac in double.  Otherwise the
 // mixed-precision step (exact index, float frac, two float64 ops per axis).
-template <int DIM, int F, bool EXACT>
-__device__ __forceinline__ bool query_prologue(const arb_grid &g, const KParams &kp, double *q,
+template <int DIM, int F, bool EXACT, typename QP>
+__device__ __forceinline__ bool query_prologue(const arb_grid &g, const KParams &kp, QP q,
                                                int64_t i, int64_t qs, int wb,
                                                const arb_query_out &o, int32_t *status,
                                                typename std::conditional<EXACT, double, float>::type frac[DIM],
                                                int64_t &idx) {
-  double *qr = q + i * qs;
+  const QP qr = q + i * qs;
   double qv[DIM];
 #pragma unroll
   for (int a = 0; a < DIM; ++a) qv[a] = qr[a];
@@ -115,8 +115,9 @@ __device__ __forceinline__ bool query_prologue(const arb_grid &g, const KParams 
   else
     s = coord_step_fast<DIM>(qv, kp.ax, g, frac);
   append_oob(o, i, s.oob);
-  if (s.oob && wb) {
-    for (int64_t c = 0; c < qs; ++c) qr[c] = qnan();
+  if constexpr (std::is_same<QP, double *>::value) {  // the caller's rows (a point comes by value)
+    if (s.oob && wb)
+      for (int64_t c = 0; c < qs; ++c) qr[c] = qnan();
   }
   if (o.inds) o.inds[i] = s.idx;
   idx = s.idx;

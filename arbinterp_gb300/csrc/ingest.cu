@@ -428,10 +428,24 @@ struct OrderWork {
   int32_t ok;
 };
 
+// The host's view of an ingest (see arb_ingest_summary).
+__device__ void write_summary(const double *axes, int64_t cap, const int64_t *count, int dim, int32_t status,
+                              double *out) {
+  out[0] = (double)status;
+  for (int a = 0; a < 4; ++a) {
+    const int64_t n = a < dim ? count[a] : 0;
+    const double nan = __longlong_as_double(0x7ff8000000000000LL);
+    out[1 + a] = (double)n;
+    out[5 + 3 * a] = n >= 1 ? axes[a * cap] : nan;
+    out[6 + 3 * a] = n >= 2 ? axes[a * cap + 1] : nan;
+    out[7 + 3 * a] = n >= 2 ? axes[a * cap + n - 2] : nan;
+  }
+}
+
 template <typename TF>
 __global__ void __launch_bounds__(256) ordered_probe_kernel(const TF *field, int64_t npts, int ncol, int dim,
                                                             int64_t cap, double *axis_out, int64_t *axis_count,
-                                                            OrderWork *w, int32_t *status) {
+                                                            OrderWork *w, int32_t *status, double *summary) {
   __shared__ long long first_stop;
   const int tid = threadIdx.x;
   if (tid == 0)  // axes the probe does not find keep a count of 0 (the caller need not clear them)
@@ -499,9 +513,15 @@ __global__ void __launch_bounds__(256) ordered_probe_kernel(const TF *field, int
     stride *= n;
   }
   if (ok && stride != npts) ok = false;
+  if (summary) __syncthreads();  // the axes are written
   if (tid == 0) {
     w->ok = ok ? 1 : 0;
-    if (!ok) set_status(status, ARB_ERR_IRREGULAR_GRID);
+    if (summary) {
+      *status = 0;
+      write_summary(axis_out, cap, axis_count, dim, ok ? 0 : ARB_ERR_IRREGULAR_GRID, summary);
+    } else if (!ok) {
+      set_status(status, ARB_ERR_IRREGULAR_GRID);
+    }
   }
 }
 
@@ -833,13 +853,13 @@ static int ordered_args_ok(const void *field, int64_t npts, int32_t ncol, int32_
 
 static void launch_ordered_probe(const void *field, int32_t field_is_f32, int64_t npts, int32_t ncol, int32_t dim,
                                  int64_t axis_cap, double *axis_out, int64_t *axis_count, OrderWork *w,
-                                 int32_t *status, cudaStream_t s) {
+                                 int32_t *status, cudaStream_t s, double *summary = nullptr) {
   if (field_is_f32)
     ordered_probe_kernel<float><<<1, 256, 0, s>>>((const float *)field, npts, ncol, dim, axis_cap, axis_out,
-                                                  axis_count, w, status);
+                                                  axis_count, w, status, summary);
   else
     ordered_probe_kernel<double><<<1, 256, 0, s>>>((const double *)field, npts, ncol, dim, axis_cap, axis_out,
-                                                   axis_count, w, status);
+                                                   axis_count, w, status, summary);
 }
 
 static int launch_ordered_fill(const void *field, int32_t field_is_f32, int64_t npts, int32_t ncol, int32_t dim,
@@ -917,16 +937,23 @@ extern "C" int arb_ingest_ordered_fill(const void *field, int32_t field_is_f32, 
 __global__ void ingest_summary_kernel(const double *axes, int64_t cap, const int64_t *count, int dim,
                                       int32_t *status, double *out) {
   if (threadIdx.x != 0) return;
-  out[0] = (double)*status;
+  write_summary(axes, cap, count, dim, *status, out);
   *status = 0;
-  for (int a = 0; a < 4; ++a) {
-    const int64_t n = a < dim ? count[a] : 0;
-    const double nan = __longlong_as_double(0x7ff8000000000000LL);
-    out[1 + a] = (double)n;
-    out[5 + 3 * a] = n >= 1 ? axes[a * cap] : nan;
-    out[6 + 3 * a] = n >= 2 ? axes[a * cap + 1] : nan;
-    out[7 + 3 * a] = n >= 2 ? axes[a * cap + n - 2] : nan;
-  }
+}
+
+// Probe and summary in one launch, on a status word that need not be cleared:
+// two launches fewer before the host knows the axes than memset, probe and
+// summary one after the other.
+extern "C" int arb_ingest_ordered_start(const void *field, int32_t field_is_f32, int64_t npts, int32_t ncol,
+                                        int32_t dim, int32_t kind, int64_t axis_cap, double *axis_out,
+                                        int64_t *axis_count, void *work, size_t work_bytes, int32_t *status,
+                                        double *summary, arb_stream_t stream) {
+  if (!axis_out || !axis_count || !work || !status || !summary) return ARB_ERR_INVALID;
+  const int rc = ordered_args_ok(field, npts, ncol, dim, kind, axis_cap, work_bytes);
+  if (rc) return rc;
+  launch_ordered_probe(field, field_is_f32, npts, ncol, dim, axis_cap, axis_out, axis_count, (OrderWork *)work,
+                       status, (cudaStream_t)stream, summary);
+  return launch_status();
 }
 
 extern "C" int arb_ingest_summary(const double *axes, int64_t axis_cap, const int64_t *axis_count, int32_t dim,

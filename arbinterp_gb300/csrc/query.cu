@@ -73,9 +73,72 @@ __global__ void __launch_bounds__(256) tab_kernel(arb_grid g, KParams kp, double
   write_vals<DIM, F>(o, i, val, grad);
 }
 
+// One point, as the row kernels evaluate it: the coordinates arrive with the
+// launch and the results go straight to pinned host memory, so a call is one
+// launch and one wait.  res: components [0..2], value [3], gradient [4..7], flat
+// cell index [8] and the status word [9] (taken and cleared) as integers.
+struct PointArg {
+  double q[4];
+};
+template <int DIM, int F, bool MIXED, bool TABLE>
+__global__ void __launch_bounds__(32) point_kernel(arb_grid g, KParams kp, PointArg p, double *res, int32_t *status) {
+  using T = typename std::conditional<MIXED, float, double>::type;
+  if (threadIdx.x) return;
+  arb_query_out o{};
+  o.comps = F >= 3 ? res : nullptr;
+  o.norms = F != 3 ? res + 3 : nullptr;
+  o.grads = F != 3 ? res + 4 : nullptr;
+  o.inds = reinterpret_cast<int64_t *>(res + 8);
+  o.comps_stride = 3;
+  o.norms_stride = 1;
+  o.grads_stride = DIM;
+  T x[DIM];
+  int64_t idx;
+  if (query_prologue<DIM, F, !MIXED>(g, kp, (const double *)p.q, 0, DIM, 0, o, status, x, idx)) {
+    int64_t c[DIM];
+    cell_coords<DIM>(idx, g, c);
+    double val[F], grad[DIM];
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) grad[a] = 0.0;
+    if constexpr (TABLE)
+      eval_tab<DIM, F, MIXED>(g, kp, c, x, val, grad);
+    else if constexpr (DIM == 3)
+      eval_otf3<F, MIXED>(g, kp, c, x, val, grad);
+    else
+      eval_otf4<F, MIXED>(g, kp, c, x, val, grad);
+    write_vals<DIM, F>(o, 0, val, grad);
+  }
+  reinterpret_cast<int64_t *>(res)[9] = atomicExch(status, 0);
+}
+
 }  // namespace arb
 
 using namespace arb;
+
+extern "C" int arb_query_point(const arb_grid *g, int32_t precision, int32_t use_table, const double *q,
+                               double *result, int32_t *status, arb_stream_t stream) {
+  if (!g || !q || !result || !status || (g->dim != 3 && g->dim != 4)) return ARB_ERR_INVALID;
+  if (g->nfield != 1 && g->nfield != 3 && g->nfield != 4) return ARB_ERR_INVALID;
+  const bool mixed = use_table ? g->table_prec == ARB_PREC_MIXED : precision == ARB_PREC_MIXED;
+  if (use_table ? !g->table : mixed ? !g->grid32 : !g->grid64) return ARB_ERR_INVALID;
+  cudaStream_t s = (cudaStream_t)stream;
+  const KParams kp = make_kparams(g);
+  PointArg p{};
+  for (int a = 0; a < g->dim; ++a) p.q[a] = q[a];
+#define PT(D, FF, MX, TB) point_kernel<D, FF, MX, TB><<<1, 32, 0, s>>>(*g, kp, p, result, status)
+#define PTF(D, MX, TB) switch (g->nfield) { case 1: PT(D, 1, MX, TB); break; case 3: PT(D, 3, MX, TB); break; default: PT(D, 4, MX, TB); break; }
+#define PTD(MX, TB) if (g->dim == 3) { PTF(3, MX, TB) } else { PTF(4, MX, TB) }
+  if (use_table) {
+    if (mixed) { PTD(true, true) } else { PTD(false, true) }
+  } else {
+    if (mixed) { PTD(true, false) } else { PTD(false, false) }
+  }
+#undef PTD
+#undef PTF
+#undef PT
+  if (cudaGetLastError() != cudaSuccess) return ARB_ERR_CUDA;
+  return cudaStreamSynchronize(s) == cudaSuccess ? ARB_OK : ARB_ERR_CUDA;
+}
 
 #define ARB_DISPATCH_F(KER, ...)                                \
   switch (g->nfield) {                                          \

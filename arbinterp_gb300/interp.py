@@ -67,6 +67,19 @@ def _probe_summary_slot(device):
     return slots[key]
 
 
+def _point_slot(device):
+    """Pinned host buffer of one point's results (arb_query_point) for this
+    thread and device: the tensor, its values and its integer view."""
+    key = torch.device(device).index
+    slots = getattr(_PER_THREAD, "point", None)
+    if slots is None:
+        slots = _PER_THREAD.point = {}
+    if key not in slots:
+        t = torch.empty(10, dtype=torch.float64, pin_memory=True)
+        slots[key] = (t, t.numpy(), t.numpy().view(np.int64))
+    return slots[key]
+
+
 def _copy_streams(device):
     """(copy-in, copy-out) side streams of a device, created once."""
     key = torch.device(device).index
@@ -238,7 +251,6 @@ class _Interpolant:
         work = torch.empty(int(wb), dtype=torch.uint8, device=dev)
         status = torch.empty(1, dtype=torch.int32, device=dev)
         s = _stream()
-        check(L.arb_status_clear(status.data_ptr(), s), "arb_status_clear")
         kind, F = self._kind, self._F
         # Mixed precision with the caller's own CUDA tensor: the float64 grid is
         # not needed by the float32 query path and is produced on first use from
@@ -269,12 +281,10 @@ class _Interpolant:
             # the grid runs while the host sets up and the first query is
             # queued, and its row check is read at the next synchronisation
             # (_settle), before any result derived from the grid is returned.
-            check(L.arb_ingest_ordered_probe(ft.data_ptr(), is32, npts, ncol, dim, kind, cap, axes.data_ptr(),
-                                             counts.data_ptr(), work.data_ptr(), wb, status.data_ptr(), s),
-                  "arb_ingest_ordered_probe")
             summ_h, ev = _probe_summary_slot(dev)
-            check(L.arb_ingest_summary(axes.data_ptr(), cap, counts.data_ptr(), dim, status.data_ptr(),
-                                       summ_h.data_ptr(), s), "arb_ingest_summary")
+            check(L.arb_ingest_ordered_start(ft.data_ptr(), is32, npts, ncol, dim, kind, cap, axes.data_ptr(),
+                                             counts.data_ptr(), work.data_ptr(), wb, status.data_ptr(),
+                                             summ_h.data_ptr(), s), "arb_ingest_ordered_start")
             ev.record()
             grid64, grid32, raw = grids()
             check(L.arb_ingest_ordered_fill(ft.data_ptr(), is32, npts, ncol, dim, kind, cap, axes.data_ptr(),
@@ -286,6 +296,8 @@ class _Interpolant:
             if done:
                 self._fill_pending = True
                 self._fill_src = (ft, is32, npts, ncol, cap, axes, counts, work, wb, grid64, grid32, raw)
+        else:
+            check(L.arb_status_clear(status.data_ptr(), s), "arb_status_clear")
         if not done:
             if grid32 is None and grid64 is None:
                 grid64, grid32, raw = grids()
@@ -695,8 +707,10 @@ class _Interpolant:
         hrows.copy_(rows, non_blocking=True)
         R, ci, ni, gi = self._row_layout()
         host = [None if c is None else hrows[:, c:c + w] for c, w in ((ci, 3), (ni, 1), (gi, dim))]
+        hcnt = torch.empty(1, dtype=torch.int64, pin_memory=True)
+        hcnt.copy_(cnt, non_blocking=True)
         st = self._fetch_status()          # synchronises the stream
-        nbad = int(cnt.item())
+        nbad = int(hcnt[0])
         if nbad:
             _nan_rows(qa, oob[:nbad].cpu())  # in-place on the caller's array
         self._last_inds = inds
@@ -783,21 +797,34 @@ class _Interpolant:
             if qv[a] < self._lo[a] or qv[a] > self._hi[a]:
                 return np.nan
         self._settle()
-        row = torch.tensor([qv], dtype=torch.float64).to(self.device)
-        comps, norms, grads, inds, _, _ = self._run(row, 1, dim, False, False)
-        st = self._fetch_status()
-        self._last_ind = inds
+        k = self._kind
+        plan = None if is_t else self._plan(None, 1, dim)
+        if plan is not None and not plan["binned"]:
+            # one launch that takes the point and leaves the results in pinned
+            # host memory (a row upload and three downloads took 4 more waits)
+            self.last_plan = plan
+            pinned, res, ints = _point_slot(self.device)
+            prec = _lib.PREC_FP64 if self.precision == "fp64" else _lib.PREC_MIXED
+            check(lib().arb_query_point(self._gs, prec, int(plan["table"]), (ctypes.c_double * 4)(*qv),
+                                        pinned.data_ptr(), self._status.data_ptr(), _stream()), "arb_query_point")
+            self._last_ind = int(ints[8])
+            st = int(ints[9])
+            c, nv, gv = res[:3].copy(), np.float64(res[3]), res[4:4 + dim].copy()
+        else:
+            row = torch.tensor([qv], dtype=torch.float64).to(self.device)
+            comps, norms, grads, inds, _, _ = self._run(row, 1, dim, False, False)
+            st = self._fetch_status()
+            self._last_ind = inds
+            if is_t:
+                c = None if comps is None else comps[0]
+                nv = None if norms is None else norms[0, 0]
+                gv = None if grads is None else grads[0]
+            else:
+                c = None if comps is None else comps[0].cpu().numpy()
+                nv = None if norms is None else np.float64(norms[0, 0].item())
+                gv = None if grads is None else grads[0].cpu().numpy()
         if st & _lib.ARB_ERR_CELL_INDEX:
             raise IndexError("cell index beyond the coefficient table (query on an upper face)")
-        k = self._kind
-        if is_t:
-            c = None if comps is None else comps[0]
-            nv = None if norms is None else norms[0, 0]
-            gv = None if grads is None else grads[0]
-        else:
-            c = None if comps is None else comps[0].cpu().numpy()
-            nv = None if norms is None else np.float64(norms[0, 0].item())
-            gv = None if grads is None else grads[0].cpu().numpy()
         if k == _lib.KIND_VECTOR:
             return c
         if k == _lib.KIND_BOTH:
@@ -878,7 +905,8 @@ class _Interpolant:
 
     @property
     def queryInd(self):
-        return None if self._last_ind is None else int(self._last_ind[0].item())
+        i = self._last_ind
+        return i if i is None or isinstance(i, int) else int(i[0].item())
 
     @property
     def A(self):

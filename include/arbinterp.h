@@ -159,6 +159,13 @@ int arb_ingest_ordered_probe(const void *field, int32_t field_is_f32, int64_t np
                              int64_t *axis_count, void *work, size_t work_bytes, int32_t *status,
                              arb_stream_t stream);
 
+/* arb_ingest_ordered_probe and arb_ingest_summary in one launch: *status need
+ * not be cleared before (it is 0 after), summary (17 doubles, host-pinned or
+ * device) as arb_ingest_summary writes it, its out[0] the probe's status. */
+int arb_ingest_ordered_start(const void *field, int32_t field_is_f32, int64_t npts, int32_t ncol, int32_t dim,
+                             int32_t kind, int64_t axis_cap, double *axis_out, int64_t *axis_count, void *work,
+                             size_t work_bytes, int32_t *status, double *summary, arb_stream_t stream);
+
 int arb_ingest_ordered_fill(const void *field, int32_t field_is_f32, int64_t npts, int32_t ncol,
                             int32_t dim, int32_t kind, int64_t axis_cap, const double *axis_out,
                             const void *work, size_t work_bytes, double *grid64, float *grid32,
@@ -205,6 +212,15 @@ int arb_query_eval(const arb_grid *g, double *q, int64_t nq, int64_t q_stride,
 int arb_query_eval_otf(const arb_grid *g, int32_t precision, double *q, int64_t nq,
                        int64_t q_stride, int32_t q_writeback, const arb_query_out *out,
                        int32_t *status, arb_stream_t stream);
+
+/* ---- one point: as arb_query_eval_otf (use_table == 0) or arb_query_eval
+ *      evaluates one row, with the coordinates in host memory and the results
+ *      in `result`, 10 doubles of pinned host memory: components [0..2], value
+ *      or |B| [3], gradient [4..7], the flat cell index [8] and the status word
+ *      [9] (taken and cleared) as int64.  Waits for the stream.  Replaces
+ *      sQuery1/2/3 (src/ARBInterp/ARBInterp.py:213-342, 916-1062). ---------- */
+int arb_query_point(const arb_grid *g, int32_t precision, int32_t use_table, const double *q, double *result,
+                    int32_t *status, arb_stream_t stream);
 
 /* ---- cell-grouped evaluation: the same contract as arb_query_eval_otf
  *      (use_table == 0) or arb_query_eval (use_table != 0, table precision
