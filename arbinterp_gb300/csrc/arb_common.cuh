@@ -93,7 +93,7 @@ __device__ __forceinline__ void hermite_slope(T t, T hb[2], T dhb[2]) {
 // be the IEEE one so floors (hence cell indices) are bit-exact.
 struct CoordStep {
   int64_t idx;       // flat cell index, as the reference computes it
-  int64_t fl[4];     // per-axis floors (valid when !oob && !nan)
+  int32_t fl[4];     // per-axis floors (valid when !oob && !nan)
   bool oob;          // some coordinate outside [lo, hi]  -> row written NaN
   bool nan;          // some coordinate NaN (row not rewritten, outputs NaN)
 };
@@ -106,6 +106,7 @@ __host__ __device__ __forceinline__ unsigned long long ord_key_bits(unsigned lon
 
 __device__ __forceinline__ void split_f32(double v, float &hi, float &lo);
 __device__ __forceinline__ void split_f32_trunc(unsigned long long b, float &hi, float &lo);
+__device__ __forceinline__ void split_f32_trunc_bits(unsigned long long b, float &hi, float &lo);
 
 // x unchanged, its origin hidden from the optimiser (no instruction): bit
 // tests on a reinterpreted double are then not turned into float64 compares.
@@ -122,6 +123,13 @@ struct FastAxis {
   unsigned long long hm, hinv;        // significand of h (53 bits) and floor(2^115 / hm), for axis_step_fx
   int he;                             // biased exponent of h; 0 where axis_step_fx does not apply
 };
+
+// Range of the axis as keys, finite so that every NaN lies outside.
+__host__ __device__ __forceinline__ void fast_axis_range(FastAxis &f, unsigned long long lo, unsigned long long hi) {
+  const unsigned long long ninf = ord_key_bits(0xfff0000000000000ULL), pinf = ord_key_bits(0x7ff0000000000000ULL);
+  f.lo_key = ord_key_bits(lo) > ninf ? ord_key_bits(lo) : ninf;
+  f.hi_key = ord_key_bits(hi) < pinf ? ord_key_bits(hi) : pinf;
+}
 
 // Constants of axis_step_fx: h normal, finite and positive.  floor(2^115 / hm)
 // by a float64 quotient (53 of its 63 bits) and two integer corrections.
@@ -188,15 +196,15 @@ __host__ __device__ inline void fast_axis_pairs(FastAxis &f, double lo, double h
 // and dividing by h could floor differently) is the IEEE division redone.
 // The float64 step of one axis: (q - IntMin) * (1/h), floored, with the
 // reference's own division where the product lands within 8 ulps of an
-// integer.  Out of line, so the float32 fast path never issues these
-// float64-pipe instructions speculatively; it is the main path only for an
-// axis spanning more than 2^20 cells.
+// integer.  Only axis_step_rest has it, out of line, so the float32 fast path
+// never issues these float64-pipe instructions speculatively; it is the main
+// path only for an axis spanning more than 2^20 cells.
 struct AxisStep {
   int64_t k;
   float fr;
 };
 
-static __device__ __noinline__ AxisStep axis_step_f64(double q, const FastAxis &ax) {
+__device__ __forceinline__ AxisStep axis_step_f64(double q, const FastAxis &ax) {
   const double d = q - ax.lo;
   double iu = d * ax.inv_h;
   const unsigned long long b = (unsigned long long)__double_as_longlong(iu);
@@ -236,7 +244,7 @@ static __device__ __noinline__ AxisStep axis_step_f64(double q, const FastAxis &
 // for bit as float64 arithmetic gives them.  The division, compares, floor and
 // conversions would be ~17 float64-pipe operations per axis at 2 lanes per SM
 // and clock (binning passes of 1e7 rows: 0.72 + 1.02 ms); here all but the
-// subtraction are integer operations (0.16 + 0.57 ms).
+// subtraction are integer operations (0.15 + 0.20 ms).
 // fx_quotient: the significand quotient md / hm by the reciprocal hinv; the
 // estimate is low by at most one, the remainder (exact modulo 2^64) corrects
 // and rounds it.  A quotient of two 53-bit significands is never halfway
@@ -291,128 +299,160 @@ __host__ __device__ __forceinline__ bool fx_quotient(unsigned long long d, unsig
   return true;
 }
 
+// q (bits) outside [lo, hi] of an axis, or NaN (whose keys lie beyond both
+// infinities'); range_kind then says which, off the common path.
+__device__ __forceinline__ bool off_axis(unsigned long long qb, const FastAxis &ax) {
+  const unsigned long long k = ord_key_bits(qb);
+  return k < ax.lo_key || k > ax.hi_key;
+}
+template <int DIM>
+__device__ __forceinline__ void range_kind(const double *qrow, const FastAxis *ax, CoordStep &s) {
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) {
+    const unsigned long long qb = (unsigned long long)__double_as_longlong(qrow[a]);
+    const bool isnan = (qb & 0x7fffffffffffffffULL) > 0x7ff0000000000000ULL;
+    s.nan |= isnan;
+    s.oob |= !isnan && off_axis(qb, ax[a]);
+  }
+}
+template <int DIM>
+__device__ __forceinline__ int64_t flat_step(const int32_t fl[4], const arb_grid &g) {
+  unsigned long long idx = (uint32_t)fl[DIM - 1];
+#pragma unroll
+  for (int a = DIM - 2; a >= 0; --a) idx = idx * (uint32_t)(g.n[a] - 3) + (uint32_t)fl[a];
+  return (int64_t)idx;
+}
+
 struct AxisStep64 {
-  double iu, k;
+  double k, frac;
 };
 static __device__ __noinline__ AxisStep64 axis_step_div(double d, double h) {
-  AxisStep64 r;
-  r.iu = d / h;
-  r.k = floor(r.iu);
+  AxisStep64 r{0.0, 0.0};
+  if (d != 0.0) {
+    const double iu = d / h;
+    r.k = floor(iu);
+    r.frac = iu - r.k;
+  }
   return r;
 }
 
+// The axes run without a branch between them; the lanes that one of them
+// leaves to the division, and the rows off the grid, take theirs after it.
 template <int DIM>
 __device__ __forceinline__ CoordStep coord_step_fx(const double *qrow, const FastAxis *ax, const arb_grid &g,
                                                    double frac[DIM]) {
   CoordStep s;
   s.oob = false;
   s.nan = false;
+  bool off = false, slow = false, fine[DIM];
 #pragma unroll
   for (int a = 0; a < DIM; ++a) {
     const double q = qrow[a];
-    const unsigned long long qb = opaque_u64((unsigned long long)__double_as_longlong(q));
-    const bool isnan = (qb & 0x7fffffffffffffffULL) > 0x7ff0000000000000ULL;
-    const unsigned long long key = ord_key_bits(qb);
-    const bool out = !isnan && (key < ax[a].lo_key || key > ax[a].hi_key);
-    s.nan |= isnan;
-    s.oob |= out;
-    s.fl[a] = 0;
-    frac[a] = 0.0;
-    if (isnan || out) continue;
+    off |= off_axis(opaque_u64((unsigned long long)__double_as_longlong(q)), ax[a]);
     const double d = __dsub_rn(q, ax[a].lo);
-    long long k;
-    unsigned long long fb;
-    if (fx_quotient(opaque_u64((unsigned long long)__double_as_longlong(d)), ax[a].hm, ax[a].hinv, ax[a].he, k, fb)) {
-      s.fl[a] = k;
-      frac[a] = __longlong_as_double((long long)fb);
-    } else if (__double_as_longlong(d) != 0) {
-      const AxisStep64 r = axis_step_div(d, ax[a].h);
-      s.fl[a] = (int64_t)r.k;
-      frac[a] = r.iu - r.k;
-    }
+    long long k = 0;
+    unsigned long long fb = 0;
+    fine[a] = fx_quotient(opaque_u64((unsigned long long)__double_as_longlong(d)), ax[a].hm, ax[a].hinv, ax[a].he, k, fb);
+    slow |= !fine[a];
+    s.fl[a] = (int32_t)k;
+    frac[a] = __longlong_as_double((long long)fb);
   }
-  if (s.oob || s.nan) {
+  if (off) {
+    range_kind<DIM>(qrow, ax, s);
     s.idx = g.nc;
     return s;
   }
-  int64_t idx = s.fl[DIM - 1];
+  if (slow) {
 #pragma unroll
-  for (int a = DIM - 2; a >= 0; --a) idx = idx * (g.n[a] - 3) + s.fl[a];
-  s.idx = idx;
+    for (int a = 0; a < DIM; ++a)
+      if (!fine[a]) {
+        const AxisStep64 r = axis_step_div(__dsub_rn(qrow[a], ax[a].lo), ax[a].h);
+        s.fl[a] = (int32_t)r.k;
+        frac[a] = r.frac;
+      }
+  }
+  s.idx = flat_step<DIM>(s.fl, g);
   return s;
 }
 
+// (q - IntMin) / h in float32 double-float arithmetic: q and IntMin as float
+// pairs (residuals 2^-47 and 2^-48 relative), an exact two-sum of the high
+// parts, times the pair of 1/h.  Error < 2^-24 in cell units (span <= 2^20
+// cells); the reference's own float64 roundings move iu by <= 2^-31.  So the
+// floor is the reference's whenever the fraction is 2^-20 or more away from a
+// cell face; false otherwise (float64 steps decide).
+__device__ __forceinline__ bool axis_step_df(float qh, float ql, const FastAxis &ax, int32_t &k, float &fr) {
+  const float sh = __fsub_rn(qh, ax.loh);
+  const float bv = __fsub_rn(sh, qh);
+  const float se = __fadd_rn(__fsub_rn(qh, __fsub_rn(sh, bv)), __fsub_rn(-ax.loh, bv));
+  const float st = __fadd_rn(se, __fsub_rn(ql, ax.lol));
+  const float ph = __fmul_rn(sh, ax.ih);
+  const float pe = __fmaf_rn(sh, ax.ih, -ph);
+  const float pl = __fmaf_rn(sh, ax.il, __fmaf_rn(st, ax.ih, pe));
+  float kf = __fsub_rn(__fadd_rd(ph, 8388608.f), 8388608.f);  // floor (0 <= ph < 2^21)
+  fr = __fadd_rn(__fsub_rn(ph, kf), pl);
+  const float up = fr < 0.f ? -1.f : fr >= 1.f ? 1.f : 0.f;
+  kf = __fadd_rn(kf, up);
+  fr = __fsub_rn(fr, up);
+  k = __float_as_int(__fadd_rn(kf, 8388608.f)) - 0x4b000000;
+  return kf >= 0.f && fr >= 0x1p-20f && fr <= 1.f - 0x1p-20f;
+}
+
+// Whatever the inline step leaves: magnitudes that float32 pairs need a
+// rounded split for, fractions by a cell face, axes without the float step.
+// (The axis by value: a reference would keep a copy of the kernel's parameters.)
+static __device__ __noinline__ AxisStep axis_step_rest(double q, FastAxis ax) {
+  AxisStep r;
+  if (ax.df) {
+    float qh, ql;
+    int32_t k;
+    split_f32_trunc((unsigned long long)__double_as_longlong(q), qh, ql);
+    if (axis_step_df(qh, ql, ax, k, r.fr)) {
+      r.k = k;
+      return r;
+    }
+  }
+  return axis_step_f64(q, ax);
+}
+
+// Branch-free over the axes as coord_step_fx, its range tests and indices on
+// 32-bit integers: 420 -> 337 instructions a row of the counting pass, 538 -> 390
+// of the placement (1.01e7 mixed rows: 132 -> 122 and 257 -> 188 us).
 template <int DIM>
 __device__ __forceinline__ CoordStep coord_step_fast(const double *qrow, const FastAxis *ax,
                                                      const arb_grid &g, float frac[DIM]) {
   CoordStep s;
   s.oob = false;
   s.nan = false;
-  int64_t fl[DIM];
+  bool off = false, slow = false, fine[DIM];
 #pragma unroll
   for (int a = 0; a < DIM; ++a) {
-    const double q = qrow[a];
-    // the bits are opaque to the optimiser, so the NaN and range tests below
-    // stay integer operations instead of being folded into float64 compares
-    // (the float64 pipe issues about one warp instruction per 15 cycles per SM)
-    const unsigned long long qb = opaque_u64((unsigned long long)__double_as_longlong(q));
-    const bool isnan = (qb & 0x7fffffffffffffffULL) > 0x7ff0000000000000ULL;
-    const unsigned long long k = ord_key_bits(qb);
-    const bool out = !isnan && (k < ax[a].lo_key || k > ax[a].hi_key);
-    s.nan |= isnan;
-    s.oob |= out;
-    if (isnan || out) {
-      fl[a] = 0;
-      frac[a] = 0.f;
-      continue;
-    }
-    if (ax[a].df) {
-      // (q - IntMin) / h in float32 double-float arithmetic: q and IntMin
-      // as float pairs (residuals 2^-47 and 2^-48 relative), an exact
-      // two-sum of the high parts, times the pair of 1/h.  Error < 2^-24 in
-      // cell units (span <= 2^20 cells); the reference's own float64
-      // roundings move iu by <= 2^-31.  So the floor is the reference's
-      // whenever the fraction is 2^-20 or more away from a cell face;
-      // otherwise the float64 steps below decide.
-      float qh, ql;
-      split_f32_trunc(qb, qh, ql);
-      const float sh = __fsub_rn(qh, ax[a].loh);
-      const float bv = __fsub_rn(sh, qh);
-      const float se = __fadd_rn(__fsub_rn(qh, __fsub_rn(sh, bv)), __fsub_rn(-ax[a].loh, bv));
-      const float st = __fadd_rn(se, __fsub_rn(ql, ax[a].lol));
-      const float ph = __fmul_rn(sh, ax[a].ih);
-      const float pe = __fmaf_rn(sh, ax[a].ih, -ph);
-      const float pl = __fmaf_rn(sh, ax[a].il, __fmaf_rn(st, ax[a].ih, pe));
-      float kf = __fsub_rn(__fadd_rn(ph, 8388608.f), 8388608.f);  // nearest integer (0 <= ph < 2^21)
-      if (kf > ph) kf = __fsub_rn(kf, 1.f);
-      float fr = __fadd_rn(__fsub_rn(ph, kf), pl);
-      if (fr < 0.f) {
-        kf = __fsub_rn(kf, 1.f);
-        fr = __fadd_rn(fr, 1.f);
-      } else if (fr >= 1.f) {
-        kf = __fadd_rn(kf, 1.f);
-        fr = __fsub_rn(fr, 1.f);
-      }
-      if (kf >= 0.f && fr >= 0x1p-20f && fr <= 1.f - 0x1p-20f) {
-        fl[a] = (int64_t)(__float_as_int(__fadd_rn(kf, 8388608.f)) - 0x4b000000);
-        frac[a] = fr;
-        continue;
-      }
-    }
-    const AxisStep r = axis_step_f64(q, ax[a]);
-    fl[a] = r.k;
-    frac[a] = r.fr;
+    // the bits are opaque to the optimiser, so the range tests stay integer
+    // operations instead of being folded into float64 compares (the float64
+    // pipe issues about one warp instruction per 15 cycles per SM)
+    const unsigned long long qb = opaque_u64((unsigned long long)__double_as_longlong(qrow[a]));
+    off |= off_axis(qb, ax[a]);
+    float qh, ql;
+    split_f32_trunc_bits(qb, qh, ql);
+    const bool in = (((uint32_t)(qb >> 52) & 0x7ffu) - 949u) <= 1149u - 949u;
+    fine[a] = axis_step_df(qh, ql, ax[a], s.fl[a], frac[a]) && in && ax[a].df;
+    slow |= !fine[a];
   }
-#pragma unroll
-  for (int a = 0; a < DIM; ++a) s.fl[a] = fl[a];
-  if (s.oob || s.nan) {
+  if (off) {
+    range_kind<DIM>(qrow, ax, s);
     s.idx = g.nc;
     return s;
   }
-  int64_t idx = fl[DIM - 1];
+  if (slow) {
 #pragma unroll
-  for (int a = DIM - 2; a >= 0; --a) idx = idx * (g.n[a] - 3) + fl[a];
-  s.idx = idx;
+    for (int a = 0; a < DIM; ++a)
+      if (!fine[a]) {
+        const AxisStep r = axis_step_rest(qrow[a], ax[a]);
+        s.fl[a] = (int32_t)r.k;
+        frac[a] = r.fr;
+      }
+  }
+  s.idx = flat_step<DIM>(s.fl, g);
   return s;
 }
 
@@ -482,7 +522,7 @@ template <int DIM>
 __device__ __forceinline__ void cell_from_step(const CoordStep &s, const arb_grid &g, int64_t c[DIM]) {
   bool face = false;
 #pragma unroll
-  for (int a = 0; a < DIM; ++a) face |= s.fl[a] >= g.n[a] - 3;
+  for (int a = 0; a < DIM; ++a) face |= s.fl[a] >= (int32_t)(g.n[a] - 3);
   if (face) {
     cell_coords<DIM>(s.idx, g, c);
   } else {

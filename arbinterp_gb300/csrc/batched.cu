@@ -22,8 +22,7 @@ __device__ void make_kparams_axis(const arb_grid &g, int a, KParams &kp) {
   const double lo = a < g.dim ? g.lo[a] : 0.0, hi = a < g.dim ? g.hi[a] : 0.0;
   kp.inv_h[a] = 1.0 / h;
   kp.inv_hf[a] = (float)(1.0 / h);
-  kp.ax[a].lo_key = ord_key_bits((unsigned long long)__double_as_longlong(lo));
-  kp.ax[a].hi_key = ord_key_bits((unsigned long long)__double_as_longlong(hi));
+  fast_axis_range(kp.ax[a], (unsigned long long)__double_as_longlong(lo), (unsigned long long)__double_as_longlong(hi));
   kp.ax[a].lo = lo;
   kp.ax[a].h = h;
   kp.ax[a].inv_h = 1.0 / h;

@@ -1130,8 +1130,7 @@ static inline KParams make_kparams(const arb_grid *g) {
     const double lo = a < g->dim ? g->lo[a] : 0.0, hi = a < g->dim ? g->hi[a] : 0.0;
     memcpy(&lb, &lo, 8);
     memcpy(&hb, &hi, 8);
-    kp.ax[a].lo_key = ord_key_bits(lb);
-    kp.ax[a].hi_key = ord_key_bits(hb);
+    fast_axis_range(kp.ax[a], lb, hb);
     kp.ax[a].lo = lo;
     kp.ax[a].h = h;
     kp.ax[a].inv_h = 1.0 / h;

@@ -220,10 +220,11 @@ static size_t carve(SortedWork *w, void *base, const arb_grid *g, int precision,
 }
 
 // Coordinate step of query row i: cell index, fraction, packed cell word
-// and bin (the special bin nbins for rows that need no evaluation).
+// and sub-bin (nsub for rows that need no evaluation).  Sub-bins are numbered
+// in 32 bits: a histogram of 2^32 counters would not fit the device.
 template <int DIM, bool EXACT, typename T>
 __device__ __forceinline__ CoordStep bin_step(const arb_grid &g, const KParams &kp, const BinGeom &bg,
-                                              const double *qr, T frac[DIM], unsigned long long &cw, int64_t &bin,
+                                              const double *qr, T frac[DIM], unsigned long long &cw, uint32_t &bin,
                                               bool &bad_index) {
   double qv[DIM];
 #pragma unroll
@@ -233,31 +234,64 @@ __device__ __forceinline__ CoordStep bin_step(const arb_grid &g, const KParams &
     s = coord_step_fx<DIM>(qv, kp.ax, g, frac);
   else
     s = coord_step_fast<DIM>(qv, kp.ax, g, frac);
-  bin = bg.nsub;
+  bin = (uint32_t)bg.nsub;
   bad_index = false;
-  if (s.oob || s.nan) {
-    cw = CELL_SPECIAL;
-  } else if (s.idx > g.nc) {
-    bad_index = true;
-    cw = CELL_SPECIAL;
-  } else if (s.idx == g.nc) {
-    cw = CELL_SPECIAL | 1ULL;
-  } else {
+  if (s.idx < g.nc) {
     int64_t c[DIM];
     cell_from_step<DIM>(s, g, c);
     cw = pack_cell<DIM>(c);
-    bin = c[DIM - 1] >> bg.shift;
+    uint32_t b = (uint32_t)c[DIM - 1] >> bg.shift;
 #pragma unroll
-    for (int a = DIM - 2; a >= 0; --a) bin = bin * bg.nb[a] + (c[a] >> bg.shift);
-    if constexpr (DIM == 3) {
-      if (bg.cls) bin = (bin << 4) | bank_class(c[0], c[1], c[2]);
-    } else {
-      if (bg.cls) bin = (bin << 4) | bank_class4(c[0], c[1], c[2], c[3]);
+    for (int a = DIM - 2; a >= 0; --a) b = b * (uint32_t)bg.nb[a] + ((uint32_t)c[a] >> bg.shift);
+    if (bg.cls) {
+      if constexpr (DIM == 3)
+        b = (b << 4) | bank_class(c[0], c[1], c[2]);
+      else
+        b = (b << 4) | bank_class4(c[0], c[1], c[2], c[3]);
     }
+    bin = b;
+  } else {
+    cw = CELL_SPECIAL;
+    bad_index = s.idx > g.nc;
+    if (!bad_index && !s.oob && !s.nan) cw |= 1ULL;
   }
   return s;
 }
 
+// One 32-byte store: a whole sector, no partial-sector merge in L2.
+__device__ __forceinline__ void store_rec32(void *dst, const void *rec) {
+  const uint32_t *u = reinterpret_cast<const uint32_t *>(rec);
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(u[0]), "r"(u[1]), "r"(u[2]),
+               "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7])
+               : "memory");
+}
+
+// Record of row i in the form of its precision.
+template <int DIM, typename T>
+__device__ __forceinline__ void store_rec(void *recs, int64_t pos, int64_t i, unsigned long long cw, int64_t idx,
+                                          T frac[DIM]) {
+  if constexpr (sizeof(T) == 4) {
+    QRec rec;
+    rec.cell = cw;
+    rec.row = (uint32_t)i;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) rec.f[a] = a < DIM ? frac[a] : 0.f;
+    rec.pad = 0;
+    store_rec32(reinterpret_cast<QRec *>(recs) + pos, &rec);
+  } else {
+    const QRec64<DIM> rec = make_rec64<DIM>((unsigned long long)idx, (uint32_t)i, frac);
+    QRec64<DIM> *dst = reinterpret_cast<QRec64<DIM> *>(recs) + pos;
+    if constexpr (DIM == 3)
+      store_rec32(dst, &rec);
+    else
+      *dst = rec;
+  }
+}
+
+// Rows that need no evaluation are stored here already, from the end of the
+// records down (the special sub-bin's place, whatever the scan will find):
+// ranked in the placement pass, one counter for all of them held that pass up
+// (1 % of 1e7 rows outside: 257 -> 198 us without them).
 template <int DIM, bool EXACT, typename T>
 __global__ void __launch_bounds__(256) bin_count_kernel(arb_grid g, KParams kp, BinGeom bg, double *q, int64_t nq,
                                                         int64_t qs, int wb, arb_query_out o, int32_t *status,
@@ -267,15 +301,26 @@ __global__ void __launch_bounds__(256) bin_count_kernel(arb_grid g, KParams kp, 
   double *qr = q + i * qs;
   T frac[DIM];
   unsigned long long cw;
-  int64_t bin;
+  uint32_t bin;
   bool bad;
   const CoordStep s = bin_step<DIM, EXACT, T>(g, kp, bg, qr, frac, cw, bin, bad);
   append_oob(o, i, s.oob);
   if (o.inds) o.inds[i] = s.idx;
+  if (bin != (uint32_t)bg.nsub) {
+    atomicAdd(&w.hist[bin], 1u);
+    return;
+  }
   if (bad) set_status(status, ARB_ERR_CELL_INDEX);
-  atomicAdd(&w.hist[bin], 1u);
+  const unsigned mask = __activemask();
+  const int lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
+  uint32_t r = 0;
+  if (lane == leader) r = atomicAdd(&w.hist[bin], (uint32_t)__popc(mask));
+  r = __shfl_sync(mask, r, leader) + __popc(mask & ((1u << lane) - 1));
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) frac[a] = T(0);
+  store_rec<DIM, T>(w.rec, nq - 1 - (int64_t)r, i, cw, (int64_t)(NAN_CELL<DIM> - (cw & 1ULL)), frac);
   // the caller's out-of-volume rows become NaN (the place pass reads them
-  // back as NaN rows: the same special bin)
+  // back as NaN rows: special all the same)
   if (s.oob && wb)
     for (int64_t c = 0; c < qs; ++c) qr[c] = qnan();
 }
@@ -297,23 +342,20 @@ __device__ __forceinline__ uint32_t bank_slot(const uint32_t o[NC + 1], int c, u
   return pos;
 }
 
-// bank_slot from a bin header: start, and the 16 class counts as bytes.
+// bank_slot from a bin header: start, and the 16 class counts n_k as bytes
+// (r < 255), two to a word of 16-bit lanes: the sum of min(n_k, r), and the
+// classes k < c with n_k > r from the carries of n_k + 255 - r.
 __device__ __forceinline__ uint32_t bank_slot_hdr(const uint32_t cnt[4], uint32_t start, int c, uint32_t r) {
-  uint32_t pos = start;
+  const uint32_t rr = r * 0x10001u, up = (255u - r) * 0x10001u;
+  uint32_t sum = 0, more = 0;
 #pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const uint32_t n = (cnt[k >> 2] >> (8 * (k & 3))) & 255u;
-    pos += min(n, r) + ((k < c && n > r) ? 1u : 0u);
+  for (int j = 0; j < 8; ++j) {  // word j >> 1: classes 4 (j >> 1) + (j & 1) and that plus 2
+    const uint32_t n = (j & 1 ? cnt[j >> 1] >> 8 : cnt[j >> 1]) & 0x00ff00ffu;
+    sum += __vminu2(n, rr);
+    more |= (((n + up) >> 8) & 0x00010001u) << (4 * (j >> 1) + (j & 1));
   }
-  return pos;
-}
-
-// One 32-byte store: a whole sector, no partial-sector merge in L2.
-__device__ __forceinline__ void store_rec32(void *dst, const void *rec) {
-  const uint32_t *u = reinterpret_cast<const uint32_t *>(rec);
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(u[0]), "r"(u[1]), "r"(u[2]),
-               "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7])
-               : "memory");
+  const uint32_t below = (1u << c) - 1u;
+  return start + (sum & 0xffffu) + (sum >> 16) + __popc(more & (below | below >> 2 << 16));
 }
 
 template <int DIM, bool EXACT, typename T>
@@ -323,13 +365,14 @@ __global__ void __launch_bounds__(256) bin_place_kernel(arb_grid g, KParams kp, 
   if (i >= nq) return;
   T frac[DIM];
   unsigned long long cw;
-  int64_t bin;
+  uint32_t bin;
   bool bad;
   const CoordStep s = bin_step<DIM, EXACT, T>(g, kp, bg, q + i * qs, frac, cw, bin, bad);
+  if (bin == (uint32_t)bg.nsub) return;  // stored by the counting pass
   // rank inside the sub-bin (any order: the count runs back down to zero)
   const uint32_t r = atomicSub(&w.hist[bin], 1u) - 1u;
   uint32_t pos;
-  if (bg.cls && bin < bg.nsub) {
+  if (bg.cls) {
     constexpr int NC = 16;  // the class sub-bins of one bin
     uint32_t h[8];
     asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -338,7 +381,7 @@ __global__ void __launch_bounds__(256) bin_place_kernel(arb_grid g, KParams kp, 
     if (!h[5]) {
       pos = bank_slot_hdr(h, h[4], (int)(bin & (NC - 1)), r);
     } else {
-      const int64_t b0 = bin & ~(int64_t)(NC - 1);
+      const uint32_t b0 = bin & ~(uint32_t)(NC - 1);
       uint32_t o[NC + 1];
 #pragma unroll
       for (int k = 0; k <= NC; ++k) o[k] = w.offs[b0 + k];
@@ -347,27 +390,7 @@ __global__ void __launch_bounds__(256) bin_place_kernel(arb_grid g, KParams kp, 
   } else {
     pos = w.offs[bin] + r;
   }
-  if constexpr (sizeof(T) == 4) {
-    QRec rec;
-    rec.cell = cw;
-    rec.row = (uint32_t)i;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) rec.f[a] = a < DIM ? frac[a] : 0.f;
-    rec.pad = 0;
-    store_rec32(reinterpret_cast<QRec *>(w.rec) + pos, &rec);
-  } else {
-    const unsigned long long cell =
-        (cw & CELL_SPECIAL) ? NAN_CELL<DIM> - (cw & 1ULL) : (unsigned long long)s.idx;
-#pragma unroll
-    for (int a = 0; a < DIM; ++a)
-      if (cw & CELL_SPECIAL) frac[a] = 0.0;
-    const QRec64<DIM> rec = make_rec64<DIM>(cell, (uint32_t)i, frac);
-    QRec64<DIM> *dst = reinterpret_cast<QRec64<DIM> *>(w.rec) + pos;
-    if constexpr (DIM == 3)
-      store_rec32(dst, &rec);
-    else
-      *dst = rec;
-  }
+  store_rec<DIM, T>(w.rec, pos, i, cw, s.idx, frac);
 }
 
 // Block totals of the histogram chunks (SCAN_CHUNK counters per block).
