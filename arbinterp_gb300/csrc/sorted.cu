@@ -626,27 +626,58 @@ struct BinTile<3> {          // (hi_x, hi_y, hi_z, 0) per point
   float4 v[TILE_PTS];
 };
 
+// The x-rows of a tile: each one's offset in points from the tile's origin and
+// its place (y in byte 0, z in 1, t in 2), worked out once per CTA.  Per point
+// the copy then takes a division by the edge and one shared load (four
+// divisions and the index of every point were 10 % of the instructions; binned
+// passes of 1e7 rows, 'both' 256^3 1089 -> 1077 us and 64^3 x 32 1917 -> 1880).
+template <int DIM, int EDGE>
+struct TileRows {
+  static constexpr int N = DIM == 3 ? EDGE * EDGE : EDGE * EDGE * EDGE;
+  uint2 row[N];
+  bool narrow;  // offsets fit 32 bits
+  __device__ __forceinline__ void fill(const arb_grid &g) {  // by the whole CTA; a barrier follows
+    const unsigned long long sy = g.n[0], sz = sy * g.n[1], st = DIM == 4 ? sz * g.n[2] : 0;
+    for (int r = threadIdx.x; r < N; r += blockDim.x) {
+      const uint32_t y = r % EDGE, z = r / EDGE % EDGE, t = r / (EDGE * EDGE);
+      row[r] = make_uint2((uint32_t)(y * sy + z * sz + t * st), y | z << 8 | t << 16);
+    }
+    if (threadIdx.x == 0) narrow = EDGE * (1 + sy + sz + st) >> 32 == 0;
+  }
+};
+
 // Copy the footprint of the bin whose tile origin is o into `t` (points
 // outside the grid are skipped: no cell of the bin reads them).
 template <int F>
-__device__ __forceinline__ void load_bin_tile(const arb_grid &g, const int o[3], BinTile<F> &t) {
+__device__ __forceinline__ void load_bin_point(const arb_grid &g, int64_t npts, int64_t p, bool next, int e,
+                                               BinTile<F> &t) {
+  if constexpr (F == 4) {
+    cp_async16(&t.hi[e], reinterpret_cast<const float4 *>(g.grid32) + p);
+    cp_async4(&t.lo2[e].x, g.grid32 + npts * 4 + p);
+    if (next) cp_async4(&t.lo2[e].y, g.grid32 + npts * 4 + p + 1);
+  } else if constexpr (F == 3) {
+    cp_async16(&t.v[e], reinterpret_cast<const float4 *>(g.grid32) + p);
+  } else {
+    cp_async8(&t.v[e], reinterpret_cast<const float2 *>(g.grid32) + p);
+  }
+}
+template <int F>
+__device__ __forceinline__ void load_bin_tile(const arb_grid &g, const int o[3], BinTile<F> &t,
+                                              const TileRows<3, TILE_EDGE> &rows) {
   const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2];
-  const int64_t npts = nx * ny * nz;
+  const int64_t npts = nx * ny * nz, p0 = (o[2] * ny + o[1]) * nx + o[0];
+  const int mx = (int)min(nx - o[0], (int64_t)TILE_EDGE), my = (int)min(ny - o[1], (int64_t)TILE_EDGE),
+            mz = (int)min(nz - o[2], (int64_t)TILE_EDGE);
+  const bool whole = mx == TILE_EDGE && my == TILE_EDGE && mz == TILE_EDGE;
+  const bool narrow = rows.narrow;
+#pragma unroll 2
   for (int e = threadIdx.x; e < TILE_PTS; e += blockDim.x) {
-    const int lx = e % TILE_EDGE, r = e / TILE_EDGE;
-    const int ly = r % TILE_EDGE, lz = r / TILE_EDGE;
-    const int64_t x = o[0] + lx, y = o[1] + ly, z = o[2] + lz;
-    if (x >= nx || y >= ny || z >= nz) continue;
-    const int64_t p = (z * ny + y) * nx + x;
-    if constexpr (F == 4) {
-      cp_async16(&t.hi[e], reinterpret_cast<const float4 *>(g.grid32) + p);
-      cp_async4(&t.lo2[e].x, g.grid32 + npts * 4 + p);
-      if (lx + 1 < TILE_EDGE && x + 1 < nx) cp_async4(&t.lo2[e].y, g.grid32 + npts * 4 + p + 1);
-    } else if constexpr (F == 3) {
-      cp_async16(&t.v[e], reinterpret_cast<const float4 *>(g.grid32) + p);
-    } else {
-      cp_async8(&t.v[e], reinterpret_cast<const float2 *>(g.grid32) + p);
-    }
+    const int r = (int)((uint32_t)e / TILE_EDGE), lx = e - r * TILE_EDGE;
+    const uint2 w = rows.row[r];
+    const int ly = w.y & 0xff, lz = w.y >> 8;
+    if (!whole && (lx >= mx || ly >= my || lz >= mz)) continue;
+    const int64_t p = p0 + lx + (narrow ? (int64_t)w.x : (lz * ny + ly) * nx);
+    load_bin_point<F>(g, npts, p, lx + 1 < mx, e, t);
   }
 }
 
@@ -706,6 +737,9 @@ __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) e
                                                                    int64_t nq, arb_query_out o, SortedWork w, uint32_t share) {
   extern __shared__ __align__(16) unsigned char binc_smem[];
   BinTile<F> *tiles = reinterpret_cast<BinTile<F> *>(binc_smem);
+  __shared__ TileRows<3, TILE_EDGE> rows;
+  rows.fill(g);
+  __syncthreads();
   const QRec *recs = reinterpret_cast<const QRec *>(w.rec);
   const BinItems items(w, bg, share);
   auto origin = [&](int64_t bb, int og[3]) {
@@ -719,12 +753,12 @@ __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) e
   uint32_t t0, t1, n0, n1;
   int64_t b = items.get(blockIdx.x, t0, t1);
   origin(b, og);
-  if (t1 > t0) load_bin_tile<F>(g, og, tiles[0]);
+  if (t1 > t0) load_bin_tile<F>(g, og, tiles[0], rows);
   cp_async_commit();
   for (int64_t it = blockIdx.x; it < items.n; it += gridDim.x) {
     b = items.get(it + gridDim.x, n0, n1);
     origin(b, on);
-    if (n1 > n0) load_bin_tile<F>(g, on, tiles[stage ^ 1]);
+    if (n1 > n0) load_bin_tile<F>(g, on, tiles[stage ^ 1], rows);
     cp_async_commit();
     cp_async_wait1();
     __syncthreads();
@@ -856,38 +890,49 @@ __device__ __forceinline__ void bin_origin4(int64_t b, const BinGeom &bg, int64_
   o[3] = b * BIN4_EDGE;
 }
 
-__device__ __forceinline__ void load_bin_tile4(const arb_grid &g, const BinGeom &bg, int64_t b, BinTile4 &t) {
+__device__ __forceinline__ void load_bin_tile4(const arb_grid &g, const BinGeom &bg, int64_t b, BinTile4 &t,
+                                               const TileRows<4, TILE4_EDGE> &rows) {
   int64_t o[4];
   bin_origin4(b, bg, o);
-  const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2], nt = g.n[3];
-  const float2 *g2 = reinterpret_cast<const float2 *>(g.grid32);
+  const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2];
+  const float2 *g2 = reinterpret_cast<const float2 *>(g.grid32) + ((o[3] * nz + o[2]) * ny + o[1]) * nx + o[0];
+  int m[4];
+  bool whole = true;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    m[a] = (int)min(g.n[a] - o[a], (int64_t)TILE4_EDGE);
+    whole &= m[a] == TILE4_EDGE;
+  }
+  const bool narrow = rows.narrow;
+#pragma unroll 4
   for (int e = threadIdx.x; e < TILE4_PTS; e += blockDim.x) {
-    int r = e;
-    const int lx = r % TILE4_EDGE;
-    r /= TILE4_EDGE;
-    const int ly = r % TILE4_EDGE;
-    r /= TILE4_EDGE;
-    const int lz = r % TILE4_EDGE, lt = r / TILE4_EDGE;
-    const int64_t x = o[0] + lx, y = o[1] + ly, z = o[2] + lz, tt = o[3] + lt;
-    if (x >= nx || y >= ny || z >= nz || tt >= nt) continue;
-    cp_async8(&t.v[e], g2 + ((tt * nz + z) * ny + y) * nx + x);
+    const int r = (int)((uint32_t)e / TILE4_EDGE), lx = e - r * TILE4_EDGE;
+    const uint2 w = rows.row[r];
+    const int ly = w.y & 0xff, lz = w.y >> 8 & 0xff, lt = w.y >> 16;
+    if (!whole && (lx >= m[0] || ly >= m[1] || lz >= m[2] || lt >= m[3])) continue;
+    cp_async8(&t.v[e], g2 + lx + (narrow ? (int64_t)w.x : ((lt * nz + lz) * ny + ly) * nx));
   }
 }
 
-__global__ void __launch_bounds__(BIN4_THREADS) eval_bin4_kernel(arb_grid g, KParams kp, BinGeom bg, int64_t nq,
+// Four CTAs of 128 registers: with the 160 that the pairs would like, three are
+// slower than the scalar form (2049 against 1816 us).
+__global__ void __launch_bounds__(BIN4_THREADS, 4) eval_bin4_kernel(arb_grid g, KParams kp, BinGeom bg, int64_t nq,
                                                                  arb_query_out o, SortedWork w, uint32_t share) {
   extern __shared__ __align__(16) unsigned char bin4_smem[];
   BinTile4 *tiles = reinterpret_cast<BinTile4 *>(bin4_smem);
+  __shared__ TileRows<4, TILE4_EDGE> rows;
+  rows.fill(g);
+  __syncthreads();
   const QRec *recs = reinterpret_cast<const QRec *>(w.rec);
   const BinItems items(w, bg, share);
   int stage = 0;
   uint32_t t0, t1, n0, n1;
   int64_t b = items.get(blockIdx.x, t0, t1);
-  if (t1 > t0) load_bin_tile4(g, bg, b, tiles[0]);
+  if (t1 > t0) load_bin_tile4(g, bg, b, tiles[0], rows);
   cp_async_commit();
   for (int64_t it = blockIdx.x; it < items.n; it += gridDim.x) {
     const int64_t bn = items.get(it + gridDim.x, n0, n1);
-    if (n1 > n0) load_bin_tile4(g, bg, bn, tiles[stage ^ 1]);
+    if (n1 > n0) load_bin_tile4(g, bg, bn, tiles[stage ^ 1], rows);
     cp_async_commit();
     cp_async_wait1();
     __syncthreads();
@@ -1128,17 +1173,20 @@ __global__ void __launch_bounds__(ADJ_THREADS) adjoint_bin_kernel(arb_grid g, KP
   const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2];
   const float ih[3] = {kp.inv_hf[0], kp.inv_hf[1], kp.inv_hf[2]};
   for (int e = threadIdx.x; e < ADJ_WARPS * TILE_PTS; e += ADJ_THREADS) gts[e] = 0.f;
+  __shared__ TileRows<3, TILE_EDGE> rows;
+  rows.fill(g);
+  __syncthreads();
   int stage = 0;
   int og[3], onx[3];
   uint32_t t0, t1, n0, n1;
   int64_t b = items.get(blockIdx.x, t0, t1);
   origin(b, og);
-  if (t1 > t0) load_bin_tile<1>(g, og, tiles[0]);
+  if (t1 > t0) load_bin_tile<1>(g, og, tiles[0], rows);
   cp_async_commit();
   for (int64_t it = blockIdx.x; it < items.n; it += gridDim.x) {
     b = items.get(it + gridDim.x, n0, n1);
     origin(b, onx);
-    if (n1 > n0) load_bin_tile<1>(g, onx, tiles[stage ^ 1]);
+    if (n1 > n0) load_bin_tile<1>(g, onx, tiles[stage ^ 1], rows);
     cp_async_commit();
     cp_async_wait1();
     __syncthreads();
