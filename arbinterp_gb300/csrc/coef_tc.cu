@@ -119,6 +119,14 @@ ARB_F32X2(fadd2, "add.rn.f32x2")
 ARB_F32X2(fsub2, "sub.rn.f32x2")
 ARB_F32X2(fmul2, "mul.rn.f32x2")
 #undef ARB_F32X2
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
 
 // Two values at once: t -> (h0, h1, 2^-SH h2 parts) with t = h0 + h1 + 2^-SH h2;
 // R1 rounds to the h1 grid (3D: 2^-11, SH = 22; 4D: 2^-10, SH = 20).
@@ -342,22 +350,30 @@ __global__ void __launch_bounds__(NT, 2) coef3_tc_kernel(const __grid_constant__
 //          even: the row stride must be a multiple of 16 bytes).
 // Grids that miss these rules, and partial solves, take coef3_tc_kernel.
 //
-// One CTA per SM, three roles working on consecutive tiles at once, each
-// hand-off an mbarrier; footprints three-deep, A tiles and accumulators
-// two-deep, one staging area (the epilogue waits for the previous tile's
-// stores to have read it):
-//   producers (8 warps): the gather of a footprint into row deltas, the
-//       per-row scale, the three-part FP16 split into an A tile; thread t
-//       owns half t >> 7 (block layers 2h, 2h+1) of row t & 127;
-//   footprint loader (one thread of warp 12): the boxes three tiles ahead,
+// One CTA per SM, roles working on consecutive tiles at once, each hand-off an
+// mbarrier; footprints three-deep, A tiles, accumulators and staging areas
+// two-deep:
+//   producers (2 x 8 warps): the gather of a footprint into row deltas, the
+//       per-row scale, the three-part FP16 split into an A tile; the groups
+//       take alternate tiles, thread t of one owns half t >> 7 (block layers
+//       2h, 2h+1) of row t & 127;
+//   footprint loader (one thread of a warp): the boxes three tiles ahead,
 //       issued as soon as the producers have gathered from the buffer;
-//   MMA issuer (one thread of warp 13): the 12 MMAs of each tile into one
+//   MMA issuer (one thread of a warp): the 12 MMAs of each tile into one
 //       of two TMEM accumulator stages (3 x 64 columns each, at columns 0
 //       and 256).  Issuing a tile's MMAs takes about 1000 cycles; with the
 //       box loads in the same thread the loads fell behind the producers;
-//   epilogue (4 warps): warp 8 + w reads TMEM lanes 32w..32w+31 (a whole
-//       row per thread), combines the three part sums, stages the rows
-//       128-byte swizzled and one thread writes them with two TMA stores.
+//   epilogue (2 x 4 warps, alternate tiles): warp w of a group reads TMEM
+//       lanes 32w..32w+31 (a whole row per thread), combines the three part
+//       sums, stages the rows 128-byte swizzled and one thread writes them
+//       with two TMA stores.
+// A tile is a chain of waits in every role (one group each and one staging
+// area: 2700 cycles, the warps idle half of them and an epilogue that waited
+// for its last stores to leave shared memory), so two of each keep the issue
+// slots at 58 % and the stores going: 112 x 96 x 101 'both' 341 -> 267 us
+// (955 MB written, 2.8 -> 3.6 TB/s); one of the two alone 308 (epilogue) or
+// no gain (producers).  Warps whose rows are all past a short tile's end skip
+// their part.
 // So the split of one tile overlaps the MMAs of the previous one and the
 // epilogue and stores of the one before, where coef3_tc runs that chain in
 // order inside each CTA.  Every wait is bounded: a wait that runs out ORs
@@ -381,39 +397,44 @@ template <>
 struct TmaShape<1> {
   static constexpr int C = 128, HX = 132, HBYTES = HX * 16 * 8, LBYTES = 0;
 };
-constexpr int FP_BYTES = 17408;  // >= every shape's HBYTES + LBYTES, a multiple of 1 KB
 
-constexpr int WS_PROD = 256;                        // producer threads (warps 0-7)
-constexpr int WS_EPI = 128;                         // epilogue threads (warps 8-11)
-constexpr int WS_WARP_FP = (WS_PROD + WS_EPI) / 32;  // warp 12: footprint loads
-constexpr int WS_WARP_MMA = WS_WARP_FP + 1;           // warp 13: MMA issue
+constexpr int WS_PG = 2, WS_EG = 2;                 // producer and epilogue groups, each on alternate tiles
+constexpr int WS_GROUP = 256;                       // threads of a producer group
+constexpr int WS_PROD = WS_PG * WS_GROUP;           // producer threads (warps 0 ..)
+constexpr int WS_EGROUP = 128;                      // threads of an epilogue group
+constexpr int WS_EPI = WS_EG * WS_EGROUP;           // epilogue threads
+constexpr int WS_WARP_FP = (WS_PROD + WS_EPI) / 32;  // footprint loads
+constexpr int WS_WARP_MMA = WS_WARP_FP + 1;           // MMA issue
 constexpr int WS_THREADS = WS_PROD + WS_EPI + 64;
 constexpr int WS_TMEM_COLS = 512;                   // two accumulator stages of 3 x 64 columns
-constexpr uint32_t BAR_PROD = 1, BAR_EPI = 2;       // named barriers of the producer and epilogue warps
+constexpr uint32_t BAR_PROD = 1, BAR_EPI = 3;       // named barriers of the producer groups (1, 2) and the epilogue's (3, 4)
 constexpr int WS_FP = 3;                            // footprint buffers: boxes three tiles ahead
 
+template <int F>
 struct WsSmem {
   unsigned char a[2][A_BYTES];             // A tiles, no-swizzle K-major (offset 0)
-  unsigned char stage[2][BOX_BYTES];       // output rows of a tile: two 128-byte swizzled boxes (1 KB aligned)
+  unsigned char stage[2][2][BOX_BYTES];    // output rows of two tiles: two 128-byte swizzled boxes each (1 KB aligned)
   unsigned char b[B_BYTES];                // B = 8 A
-  unsigned char fp[WS_FP][FP_BYTES];       // footprints
-  float amax[2][2][TM];                    // [tile parity][half][row]
+  unsigned char fp[WS_FP][TmaShape<F>::HBYTES + TmaShape<F>::LBYTES];  // footprints
+  int16_t hexp[4][2][TM];                  // scale exponents of half rows: [tile mod 4][half][row]
   float mrhi[4][TM], mrlo[4][TM];          // each row's corner value (hi, lo), by tile mod 4
   int mexp[4][TM];                         // each row's scale exponent
   uint64_t fp_full[WS_FP], fp_empty[WS_FP], a_full[2], a_empty[2], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort;
 };
-static_assert(TmaShape<4>::HBYTES + TmaShape<4>::LBYTES <= FP_BYTES && TmaShape<3>::HBYTES <= FP_BYTES &&
-                  TmaShape<1>::HBYTES <= FP_BYTES,
-              "footprint buffer");
-static_assert(offsetof(WsSmem, stage) % 1024 == 0 && offsetof(WsSmem, fp) % 1024 == 0 &&
-                  offsetof(WsSmem, b) % 1024 == 0,
+static_assert(offsetof(WsSmem<1>, stage) % 1024 == 0 && offsetof(WsSmem<1>, b) % 1024 == 0 &&
+                  offsetof(WsSmem<1>, fp) % 1024 == 0,
               "alignment");
+static_assert(sizeof(WsSmem<1>::fp[0]) % 128 == 0 && sizeof(WsSmem<3>::fp[0]) % 128 == 0 &&
+                  sizeof(WsSmem<4>::fp[0]) % 128 == 0 && TmaShape<4>::HBYTES % 128 == 0,
+              "box alignment");
+static_assert(sizeof(WsSmem<1>) + 1024 <= 227 * 1024, "shared memory");
 
 // Bounded wait that also gives up once another role has raised the abort
 // flag; a wait that runs out raises it.
-__device__ __forceinline__ bool ws_wait(WsSmem &sm, uint64_t *bar, uint32_t parity, uint32_t limit,
+template <class SM>
+__device__ __forceinline__ bool ws_wait(SM &sm, uint64_t *bar, uint32_t parity, uint32_t limit,
                                         int32_t *status) {
   for (uint32_t it = 0; it < limit; ++it) {
     if (tc::mbar_try_wait(bar, parity)) return true;
@@ -433,7 +454,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
                                                                   arb_grid g, int32_t *status) {
   using S = TmaShape<F>;
   extern __shared__ unsigned char smem_raw[];
-  WsSmem &sm = smem_aligned_1k<WsSmem>(smem_raw);
+  WsSmem<F> &sm = smem_aligned_1k<WsSmem<F>>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t ncx = g.n[0] - 3, ncy = g.n[1] - 3, ncz = g.n[2] - 3;
   const int64_t tpr = (ncx + S::C - 1) / S::C;          // tiles per x-row of cells
@@ -453,13 +474,13 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
   if (tid == 0) {
     for (int s = 0; s < WS_FP; ++s) {
       tc::mbar_init(&sm.fp_full[s], 1);
-      tc::mbar_init(&sm.fp_empty[s], WS_PROD / 32);
+      tc::mbar_init(&sm.fp_empty[s], WS_GROUP / 32);
     }
     for (int s = 0; s < 2; ++s) {
-      tc::mbar_init(&sm.a_full[s], WS_PROD / 32);
+      tc::mbar_init(&sm.a_full[s], WS_GROUP / 32);
       tc::mbar_init(&sm.a_empty[s], 1);
       tc::mbar_init(&sm.acc_full[s], 1);
-      tc::mbar_init(&sm.acc_empty[s], WS_EPI / 32);
+      tc::mbar_init(&sm.acc_empty[s], WS_EGROUP / 32);
     }
     sm.abort = 0;
     tc::fence_mbar_init();
@@ -473,10 +494,11 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
 
   if (warp < WS_PROD / 32) {
     // ---- producers: gather, scale, split -----------------------------------
-    const int row = tid & (TM - 1), half = tid >> 7;
+    const int row = tid & (TM - 1), half = (tid >> 7) & 1;
+    const int group = tid / WS_GROUP;
     const int cl = row / F, f = row % F;                 // this row's cell in the tile, and field
     bool fail = false;
-    for (int k = 0; k < nloc; ++k) {
+    for (int k = group; k < nloc; k += WS_PG) {
       const int s = k & 1;
       const uint32_t ph = (uint32_t)(k >> 1) & 1u;
       const int64_t tile = tile_of(k);
@@ -484,6 +506,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
       const int x0 = (int)((tile - xr * tpr) * S::C);
       const int cnt = tile - xr * tpr == tpr - 1 ? rem : S::C;
       const int fs = k % WS_FP;
+      const bool live = (row & ~31) < cnt * F;           // some row of this warp is in the table
       bool ok = !fail && ws_wait(sm, &sm.fp_full[fs], (uint32_t)(k / WS_FP) & 1u, WAIT_LIMIT, status);
       float rhi = 0.f, rlo = 0.f, d[32], amax = 0.f;
 #pragma unroll
@@ -525,12 +548,13 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
       }
       __syncwarp();
       if (ok && lane == 0) tc::mbar_arrive(&sm.fp_empty[fs]);  // this warp has read the footprint
-      sm.amax[s][half][row] = amax;
-      if (tc::named_bar_or(BAR_PROD, WS_PROD, !ok)) break;   // every producer leaves together
-      const int E = scale_exp(fmaxf(amax, sm.amax[s][half ^ 1][row]));
+      const int Eh = scale_exp(amax);
+      sm.hexp[k & 3][half][row] = (int16_t)Eh;
+      if (tc::named_bar_or(BAR_PROD + group, WS_GROUP, !ok)) break;  // a group leaves together
+      const int E = max(Eh, (int)sm.hexp[k & 3][half ^ 1][row]);
       const float c10 = __uint_as_float((uint32_t)(137 - E) << 23);    // 2^(10 - E)
       ok = k < 2 || ws_wait(sm, &sm.a_empty[s], ph ^ 1u, WAIT_LIMIT, status);  // the MMAs of tile k - 2 are done
-      if (ok) {
+      if (ok && live) {
         unsigned char *at = sm.a[s];
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) {
@@ -562,17 +586,19 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
     }
   } else if (warp < (WS_PROD + WS_EPI) / 32) {
     // ---- epilogue: TMEM -> table rows ----------------------------------------
-    const int ew = warp - WS_PROD / 32;                  // TMEM lanes 32 ew .. 32 ew + 31
+    const int ew = warp & 3;                             // TMEM lanes 32 ew .. 32 ew + 31
+    const int group = (tid - WS_PROD) / WS_EGROUP;
+    const bool storer = (tid - WS_PROD) % WS_EGROUP == 0;
     const int row = ew * 32 + lane;
     const uint32_t mma_wait_limit = g_mma_wait_limit;
     bool fail = false;
-    for (int k = 0; k < nloc; ++k) {
+    for (int k = group; k < nloc; k += WS_EG) {
       const int s = k & 1;
       const uint32_t ph = (uint32_t)(k >> 1) & 1u;
       const bool ok = !fail && ws_wait(sm, &sm.acc_full[s], ph, mma_wait_limit, status);
       tc::tc_fence_after();
-      if (tid == WS_PROD) tc::bulk_wait_read0();          // the stores of tile k - 1 have read the staging
-      if (tc::named_bar_or(BAR_EPI, WS_EPI, !ok)) break;
+      if (storer) tc::bulk_wait_read0();                  // the stores of tile k - 2 have read the staging
+      if (tc::named_bar_or(BAR_EPI + group, WS_EGROUP, !ok)) break;
       const int64_t tile = tile_of(k);
       const int64_t xr = tile / tpr;
       const int64_t kx = tile - xr * tpr;
@@ -582,6 +608,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
       const float rhi = sm.mrhi[k & 3][row], rlo = sm.mrlo[k & 3][row];
       const float so = __uint_as_float((uint32_t)(E - 13 + 127) << 23);   // 2^(E - 13)
       const uint32_t t_row = tmem + ((uint32_t)(ew * 32) << 16) + (uint32_t)(256 * s);
+      if (32 * ew < cnt * F)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {                      // coefficients 16q .. 16q + 15
         float p0[16], p1[16], p2[16];
@@ -590,9 +617,16 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
         tc::tmem_ld16(t_row + (uint32_t)(128 + 16 * q), p2);
         tc::tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) p0[j] = __fmul_rn(__fadd_rn(p0[j], __fmaf_rn(p2[j], 0x1p-22f, p1[j])), so);
+        for (int j = 0; j < 16; j += 2) {
+          const float2 v = fmul2(fadd2(make_float2(p0[j], p0[j + 1]),
+                                       ffma2(make_float2(p2[j], p2[j + 1]), make_float2(0x1p-22f, 0x1p-22f),
+                                             make_float2(p1[j], p1[j + 1]))),
+                                 make_float2(so, so));
+          p0[j] = v.x;
+          p0[j + 1] = v.y;
+        }
         if (q == 0) p0[0] = rhi + (rlo + p0[0]);
-        unsigned char *st_row = sm.stage[q >> 1] + row * 128;
+        unsigned char *st_row = sm.stage[s][q >> 1] + row * 128;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const int j = (q & 1) * 4 + c;                 // 16-byte chunk of the 128-byte row
@@ -604,15 +638,15 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&sm.acc_empty[s]);  // this warp has read the accumulator
       tc::fence_proxy_async_smem();
-      tc::named_bar_sync(BAR_EPI, WS_EPI);
-      if (tid == WS_PROD) {
+      tc::named_bar_sync(BAR_EPI + group, WS_EGROUP);
+      if (storer) {
         const CUtensorMap *tm = cnt == S::C ? &tmap_full : &tmap_part;
-        tc::tma_store_2d(tm, sm.stage[0], 0, (int32_t)row0);
-        tc::tma_store_2d(tm, sm.stage[1], 32, (int32_t)row0);
+        tc::tma_store_2d(tm, sm.stage[s][0], 0, (int32_t)row0);
+        tc::tma_store_2d(tm, sm.stage[s][1], 32, (int32_t)row0);
         tc::bulk_commit();
       }
     }
-    if (tid == WS_PROD) tc::bulk_wait0();
+    if (storer) tc::bulk_wait0();
   } else if (warp == WS_WARP_FP && lane == 0) {
     // ---- footprint loader: boxes WS_FP tiles ahead ---------------------------
     auto issue_fp = [&](int k) {
@@ -724,7 +758,7 @@ static int coef3_solve_tma(const arb_grid *g, float *table, int32_t *status, cud
   const int64_t ncx = nx - 3;
   const int64_t tpr = (ncx + S::C - 1) / S::C;
   const int rem = (int)(ncx - (tpr - 1) * S::C);
-  const size_t smem = sizeof(WsSmem) + 1024;
+  const size_t smem = sizeof(WsSmem<F>) + 1024;
   static std::once_flag once[MAX_DEVICES];
   static int per_sm_dev[MAX_DEVICES];
   static cudaError_t attr_err[MAX_DEVICES];
