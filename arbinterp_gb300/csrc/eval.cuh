@@ -1041,11 +1041,10 @@ static __device__ __noinline__ EvalOut<1, 4> eval_otf4_full(Grid4Ref r, EvalArgs
   FxGrid4 src;
   r.block(src, in.c);
   if (!src.scale<true>()) return eval_otf4_f64(r.grid, r.nx, r.ny, r.nz, r.F, r.f, GRADF, in);
-  FxW w[4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a) fx_axis<2>(fx_bits(in.frac[a]), w[a]);
+  FxW w[2];
+  fx_weights4(in.frac, w);
   long long R, G[4];
-  fx_eval4<GRADF>(src, w, R, G);
+  fx_eval4<GRADF>(src, w, FxZT(), R, G);
   EvalOut<1, 4> o;
   o.val[0] = fx_to_double(R, src.emax);
 #pragma unroll
@@ -1074,13 +1073,13 @@ __device__ __forceinline__ void eval_otf4_slow(const arb_grid &g, const KParams 
 // Field f of a 4D block in float64 results: as eval_otf3_fx.
 template <bool GRADF>
 __device__ __forceinline__ void eval_otf4_fx(const arb_grid &g, const KParams &kp, int F, int f, const int64_t c[4],
-                                             const FxW w[4], const double frac[4], double &val, double grad[4]) {
+                                             const FxW w[2], const double frac[4], double &val, double grad[4]) {
   FxGrid4 src;
   Grid4Ref{g.grid64, g.n[0], g.n[1], g.n[2], F, f}.block(src, c);
   bool ok = src.scale<false>();
   if (ok) {
     long long R, G[4];
-    fx_eval4<GRADF>(src, w, R, G);
+    fx_eval4<GRADF>(src, w, FxZT(), R, G);
     val = fx_to_double(R, src.emax);
     if (GRADF) {
 #pragma unroll
@@ -1098,9 +1097,8 @@ __device__ __forceinline__ void eval_otf4(const arb_grid &g, const KParams &kp, 
   if constexpr (MIXED) {
     eval_otf4_mixed<F>(g, kp, c, frac, val, grad);
   } else {
-    FxW w[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) fx_axis<2>(fx_bits(frac[a]), w[a]);
+    FxW w[2];
+    fx_weights4(frac, w);
     constexpr int NV = F == 3 ? 3 : F - 1;  // value-only fields come first
 #pragma unroll 1
     for (int f = 0; f < NV; ++f) {

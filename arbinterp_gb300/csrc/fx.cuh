@@ -155,6 +155,33 @@ __host__ __device__ __forceinline__ void fx_axis(unsigned long long tbits, FxW &
   fx_split(d3, o.dh[3], o.dl[3]);
 }
 
+// One weight of an axis and its derivative weight.
+struct FxWord {
+  int wh, wl, dh, dl;
+};
+#ifdef __CUDACC__
+// Weights of the z (0) and t (1) axes of a 4D block in shared memory, a column a
+// thread: in registers they were 32 of the ~190 that fx_eval4 has alive, and the
+// loops over k and t picked from them by selects (1.5e6 scalar queries on 33 x 41
+// x 29 x 17, one lane a query: 1122 -> 1049 us).  Kernels with 4D float64
+// evaluators have at most FX_ZT_THREADS threads.
+constexpr int FX_ZT_THREADS = 128;
+struct FxZT {
+  static __device__ __forceinline__ int4 *column() {
+    __shared__ int4 zt[8 * FX_ZT_THREADS];
+    return zt + threadIdx.x;
+  }
+  static __device__ __forceinline__ void set(int axis, const FxW &w) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) column()[(4 * axis + k) * FX_ZT_THREADS] = make_int4(w.wh[k], w.wl[k], w.dh[k], w.dl[k]);
+  }
+  __device__ __forceinline__ FxWord get(int axis, int k) const {
+    const int4 v = column()[(4 * axis + k) * FX_ZT_THREADS];
+    return FxWord{v.x, v.y, v.z, v.w};
+  }
+};
+#endif
+
 template <typename T>
 __host__ __device__ __forceinline__ T fx_sel(const T v[4], int k) {
   return k == 0 ? v[0] : (k == 1 ? v[1] : (k == 2 ? v[2] : v[3]));
@@ -241,8 +268,9 @@ __host__ __device__ __forceinline__ void fx_eval3(const SRC &src, const FxW &wx,
 // SRC::UNROLL: planes of a slab unrolled (words from a tile) or in a loop (with
 // the conversions of a gathered block the body would outgrow the instruction
 // cache).
-template <bool GRADF, class SRC>
-__host__ __device__ __forceinline__ void fx_eval4(const SRC &src, const FxW w[4], long long &R, long long G[4]) {
+template <bool GRADF, class SRC, class ZT>
+__host__ __device__ __forceinline__ void fx_eval4(const SRC &src, const FxW w[2], const ZT &zt, long long &R,
+                                                  long long G[4]) {
   FxAcc<3> V, gt;
   FxAcc<2> gx, gy, gz;
   long long S[16];
@@ -288,16 +316,16 @@ __host__ __device__ __forceinline__ void fx_eval4(const SRC &src, const FxW w[4]
           yx.mac(h, l, w[1].wh[j], w[1].wl[j]);
         }
       }
-      const int wh = fx_sel(w[2].wh, k), wl = fx_sel(w[2].wl, k);
+      const FxWord wz = zt.get(0, k);
       int h, l;
       Y.norm(h, l);
-      Z.mac(h, l, wh, wl);
+      Z.mac(h, l, wz.wh, wz.wl);
       if (GRADF) {
-        zz.mac(h, l, fx_sel(w[2].dh, k), fx_sel(w[2].dl, k));
+        zz.mac(h, l, wz.dh, wz.dl);
         yx.norm(h, l);
-        zx.mac(h, l, wh, wl);
+        zx.mac(h, l, wz.wh, wz.wl);
         yy.norm(h, l);
-        zy.mac(h, l, wh, wl);
+        zy.mac(h, l, wz.wh, wz.wl);
       }
       const long long up = k >= 2 ? 0 : -1, even = (k & 1) - 1;
 #pragma unroll
@@ -308,18 +336,18 @@ __host__ __device__ __forceinline__ void fx_eval4(const SRC &src, const FxW w[4]
         E2[m + 4] += v & ~even;
       }
     }
-    const int wh = fx_sel(w[3].wh, t), wl = fx_sel(w[3].wl, t);
+    const FxWord wt = zt.get(1, t);
     int h, l;
     Z.norm(h, l);
-    V.mac(h, l, wh, wl);
+    V.mac(h, l, wt.wh, wt.wl);
     if (GRADF) {
-      gt.mac(h, l, fx_sel(w[3].dh, t), fx_sel(w[3].dl, t));
+      gt.mac(h, l, wt.dh, wt.dl);
       zx.norm(h, l);
-      gx.mac(h, l, wh, wl);
+      gx.mac(h, l, wt.wh, wt.wl);
       zy.norm(h, l);
-      gy.mac(h, l, wh, wl);
+      gy.mac(h, l, wt.wh, wt.wl);
       zz.norm(h, l);
-      gz.mac(h, l, wh, wl);
+      gz.mac(h, l, wt.wh, wt.wl);
     }
     const long long up = t >= 2 ? 0 : -1, even = (t & 1) - 1;
 #pragma unroll
@@ -369,29 +397,31 @@ __host__ __device__ __forceinline__ void fx_eval4(const SRC &src, const FxW w[4]
     }
   }
   FxAcc<3> c0, cx, cy, cz, ct;
+  const FxWord z0 = zt.get(0, 0), z3 = zt.get(0, 3);
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
     FxAcc<2> a, b, c, d;
     int h, l;
-    const int sg = m ? 1 : -1, q = m ? 3 : 0;
-    a.mac(-Yh[2 * m], -Yl[2 * m], w[2].wh[0], w[2].wl[0]);
-    a.mac(Yh[2 * m + 1], Yl[2 * m + 1], w[2].wh[3], w[2].wl[3]);
+    const int sg = m ? 1 : -1;
+    const FxWord u = zt.get(1, m ? 3 : 0);
+    a.mac(-Yh[2 * m], -Yl[2 * m], z0.wh, z0.wl);
+    a.mac(Yh[2 * m + 1], Yl[2 * m + 1], z3.wh, z3.wl);
     a.norm(h, l);
-    c0.mac(sg * h, sg * l, w[3].wh[q], w[3].wl[q]);
+    c0.mac(sg * h, sg * l, u.wh, u.wl);
     if (GRADF) {
-      ct.mac(sg * h, sg * l, w[3].dh[q], w[3].dl[q]);
-      b.mac(-Xh[2 * m], -Xl[2 * m], w[2].wh[0], w[2].wl[0]);
-      b.mac(Xh[2 * m + 1], Xl[2 * m + 1], w[2].wh[3], w[2].wl[3]);
+      ct.mac(sg * h, sg * l, u.dh, u.dl);
+      b.mac(-Xh[2 * m], -Xl[2 * m], z0.wh, z0.wl);
+      b.mac(Xh[2 * m + 1], Xl[2 * m + 1], z3.wh, z3.wl);
       b.norm(h, l);
-      cx.mac(sg * h, sg * l, w[3].wh[q], w[3].wl[q]);
-      c.mac(-Gh[2 * m], -Gl[2 * m], w[2].wh[0], w[2].wl[0]);
-      c.mac(Gh[2 * m + 1], Gl[2 * m + 1], w[2].wh[3], w[2].wl[3]);
+      cx.mac(sg * h, sg * l, u.wh, u.wl);
+      c.mac(-Gh[2 * m], -Gl[2 * m], z0.wh, z0.wl);
+      c.mac(Gh[2 * m + 1], Gl[2 * m + 1], z3.wh, z3.wl);
       c.norm(h, l);
-      cy.mac(sg * h, sg * l, w[3].wh[q], w[3].wl[q]);
-      d.mac(-Yh[2 * m], -Yl[2 * m], w[2].dh[0], w[2].dl[0]);
-      d.mac(Yh[2 * m + 1], Yl[2 * m + 1], w[2].dh[3], w[2].dl[3]);
+      cy.mac(sg * h, sg * l, u.wh, u.wl);
+      d.mac(-Yh[2 * m], -Yl[2 * m], z0.dh, z0.dl);
+      d.mac(Yh[2 * m + 1], Yl[2 * m + 1], z3.dh, z3.dl);
       d.norm(h, l);
-      cz.mac(sg * h, sg * l, w[3].wh[q], w[3].wl[q]);
+      cz.mac(sg * h, sg * l, u.wh, u.wl);
     }
   }
   R = V.value() + c0.value();
@@ -555,6 +585,19 @@ struct FxGrid4 {
 
 __device__ __forceinline__ unsigned long long fx_bits(double v) {
   return opaque_u64((unsigned long long)__double_as_longlong(v));
+}
+
+// Weights of a 4D block: x and y in registers, z and t in shared memory.
+__device__ __forceinline__ void fx_weights4(const double frac[4], FxW w[2]) {
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    FxW v;
+    fx_axis<2>(fx_bits(frac[a]), v);
+    if (a < 2)
+      w[a] = v;
+    else
+      FxZT::set(a - 2, v);
+  }
 }
 
 // Values and gradient of a 3D block from its contraction (fx_eval3's units).

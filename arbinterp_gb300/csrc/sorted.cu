@@ -552,7 +552,7 @@ struct BinItems {
 };
 
 template <int DIM, int F, bool MIXED, bool TABLE>
-__global__ void __launch_bounds__(DIM == 3 ? 256 : 128, MIXED ? 0 : (DIM == 3 ? 2 : 3)) eval_sorted_kernel(arb_grid g, KParams kp,
+__global__ void __launch_bounds__(DIM == 3 ? 256 : 128, MIXED ? 0 : (DIM == 3 || F == 4 ? 2 : 3)) eval_sorted_kernel(arb_grid g, KParams kp,
                                                                            int64_t nq, arb_query_out o,
                                                                            SortedWork w) {
   using T = typename std::conditional<MIXED, float, double>::type;
@@ -1008,7 +1008,8 @@ static void launch_bin(const arb_grid *g, const KParams &kp, const BinGeom &bg, 
   const unsigned B = (unsigned)((nq + TB - 1) / TB);
   bin_count_kernel<DIM, !MIXED, T><<<B, TB, 0, s>>>(*g, kp, bg, q, nq, qs, wb, *out, status, w);
   const int64_t nh = bg.nsub + 1, nb = scan_blocks(nh);
-  scan_part_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(w.hist, nh, w.part);
+  // a scan of one block has no blocks before it
+  if (nb > 1) scan_part_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(w.hist, nh, w.part);
   scan_apply_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(w.hist, nh, w.part, w.offs, w.hdr, bg.nbins);
   bin_place_kernel<DIM, !MIXED, T><<<B, TB, 0, s>>>(*g, kp, bg, q, nq, qs, w);
   if (bg.cls) split_kernel<<<(unsigned)((bg.nbins + 255) / 256), 256, 0, s>>>(w.offs, bg, split_share(bg, nq), w.hist);
