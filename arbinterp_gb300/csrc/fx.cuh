@@ -26,8 +26,21 @@ namespace arb {
 constexpr int FX_DB = 61;                    // |sample| < 2^FX_DB
 constexpr int FX_EMIN = 64, FX_EMAX = 2040;  // biased exponents of the largest sample that the scaling holds
 
+// One weight of an axis and its derivative weight.
+struct FxWord {
+  int wh, wl, dh, dl;
+};
+
+template <typename T>
+__host__ __device__ __forceinline__ T fx_sel(const T v[4], int k) {
+  return k == 0 ? v[0] : (k == 1 ? v[1] : (k == 2 ? v[2] : v[3]));
+}
+
 struct FxW {  // one axis: weights w and derivative weights d (times 2^-DS), times 2^62, as words
   int wh[4], wl[4], dh[4], dl[4];
+  __host__ __device__ __forceinline__ FxWord get(int, int k) const {
+    return FxWord{fx_sel(wh, k), fx_sel(wl, k), fx_sel(dh, k), fx_sel(dl, k)};
+  }
 };
 
 // acc + a b: one IMAD.WIDE.  In PTX, because a product of words that come from
@@ -155,20 +168,17 @@ __host__ __device__ __forceinline__ void fx_axis(unsigned long long tbits, FxW &
   fx_split(d3, o.dh[3], o.dl[3]);
 }
 
-// One weight of an axis and its derivative weight.
-struct FxWord {
-  int wh, wl, dh, dl;
-};
 #ifdef __CUDACC__
-// Weights of the z (0) and t (1) axes of a 4D block in shared memory, a column a
-// thread: in registers they were 32 of the ~190 that fx_eval4 has alive, and the
+// Weights of outer axes (4D: z and t; z of the 3D 'both' tiles) in shared memory, a
+// column a thread: in registers they were 32 of the ~190 that fx_eval4 has alive, and the
 // loops over k and t picked from them by selects (1.5e6 scalar queries on 33 x 41
-// x 29 x 17, one lane a query: 1122 -> 1049 us).  Kernels with 4D float64
-// evaluators have at most FX_ZT_THREADS threads.
+// x 29 x 17, one lane a query: 1122 -> 1049 us).  Kernels that use them have at
+// most FX_ZT_THREADS threads.
 constexpr int FX_ZT_THREADS = 128;
-struct FxZT {
+template <int AXES>
+struct FxZTCols {
   static __device__ __forceinline__ int4 *column() {
-    __shared__ int4 zt[8 * FX_ZT_THREADS];
+    __shared__ int4 zt[4 * AXES * FX_ZT_THREADS];
     return zt + threadIdx.x;
   }
   static __device__ __forceinline__ void set(int axis, const FxW &w) {
@@ -180,12 +190,9 @@ struct FxZT {
     return FxWord{v.x, v.y, v.z, v.w};
   }
 };
+using FxZT = FxZTCols<2>;  // 4D: z, t
+using FxZ = FxZTCols<1>;   // 3D: z
 #endif
-
-template <typename T>
-__host__ __device__ __forceinline__ T fx_sel(const T v[4], int k) {
-  return k == 0 ? v[0] : (k == 1 ? v[1] : (k == 2 ? v[2] : v[3]));
-}
 
 // Tricubic contraction of a 4x4x4 block of F fields: R[f] the values and (F
 // != 3) G[a] the last field's derivatives times 2^-1, in the fields' units.
@@ -195,8 +202,8 @@ __host__ __device__ __forceinline__ T fx_sel(const T v[4], int k) {
 // 8 dependent IMAD.WIDE, and at three warps per scheduler the chains have to
 // hide each other's latency: the sums of RB rows and all fields advance
 // together, point by point.
-template <int F, class SRC>
-__host__ __device__ __forceinline__ void fx_eval3(const SRC &src, const FxW &wx, const FxW &wy, const FxW &wz,
+template <int F, class SRC, class WY, class WZ>
+__host__ __device__ __forceinline__ void fx_eval3(const SRC &src, const FxW &wx, const WY &wy, const WZ &wz,
                                                   long long R[F], long long G[3]) {
   constexpr bool GRAD = F != 3;
   constexpr int RB = F == 4 ? 1 : (F == 3 ? 2 : 4);
@@ -219,33 +226,33 @@ __host__ __device__ __forceinline__ void fx_eval3(const SRC &src, const FxW &wx,
         }
 #pragma unroll
       for (int r = 0; r < RB; ++r) {
-        const int j = jb + r;
+        const FxWord v = wy.get(0, jb + r);
         int h = 0, l = 0;
 #pragma unroll
         for (int f = 0; f < F; ++f) {
           a[r][f].norm(h, l);
-          Y[f].mac(h, l, wy.wh[j], wy.wl[j]);
+          Y[f].mac(h, l, v.wh, v.wl);
         }
         if (GRAD) {
-          yy.mac(h, l, wy.dh[j], wy.dl[j]);
+          yy.mac(h, l, v.dh, v.dl);
           d[r].norm(h, l);
-          yx.mac(h, l, wy.wh[j], wy.wl[j]);
+          yx.mac(h, l, v.wh, v.wl);
         }
       }
     }
-    const int wh = fx_sel(wz.wh, k), wl = fx_sel(wz.wl, k);
+    const FxWord u = wz.get(0, k);
     int h = 0, l = 0;
 #pragma unroll
     for (int f = 0; f < F; ++f) {
       Y[f].norm(h, l);
-      V[f].mac(h, l, wh, wl);
+      V[f].mac(h, l, u.wh, u.wl);
     }
     if (GRAD) {
-      gz.mac(h, l, fx_sel(wz.dh, k), fx_sel(wz.dl, k));
+      gz.mac(h, l, u.dh, u.dl);
       yx.norm(h, l);
-      gx.mac(h, l, wh, wl);
+      gx.mac(h, l, u.wh, u.wl);
       yy.norm(h, l);
-      gy.mac(h, l, wh, wl);
+      gy.mac(h, l, u.wh, u.wl);
     }
   }
 #pragma unroll

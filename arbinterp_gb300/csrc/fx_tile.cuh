@@ -22,10 +22,10 @@
 namespace arb {
 
 // Bound by the IMAD.WIDE pipe (4 cycles a warp instruction and scheduler; 'both'
-// takes 1332 of them a query, 61 % of its cycles at 305 queries a bin) and by the
+// takes 1332 of them a query, half of its cycles at 305 queries a bin) and by the
 // dependent issue of its chains at 12 to 16 warps per SM.  Three CTAs of 128
-// threads and 168 registers for 'both' (four of 128 with spills 3418 against 3276 us
-// for the binned pass of 1e7 on 256^3; 96, 160, 192 or 256 threads 3447-3636).
+// threads and 168 registers for 'both' (four of 128 with spills 3222 against 3097 us
+// for the binned pass of 1e7 on 256^3; 96, 160, 192 or 256 threads were 5-11 % slower).
 constexpr int FX_THREADS = 128;
 constexpr int FX_EVEN3 = 5, FX_EVEN4 = 5;
 
@@ -291,12 +291,19 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
         fx_axis<1>(fx_bits(fr[0]), wx);
         fx_axis<1>(fx_bits(fr[1]), wy);
         fx_axis<1>(fx_bits(fr[2]), wz);
+        auto eval = [&](const auto &src, long long R[F], long long G[3]) {
+          if constexpr (F == 4)  // z weights from shared memory: 3215 -> 3097 us, with y's too 3092
+            fx_eval3<F>(src, wx, wy, FxZ(), R, G);
+          else
+            fx_eval3<F>(src, wx, wy, wz, R, G);
+        };
+        if constexpr (F == 4) FxZ::set(0, wz);
         long long R[F], G[3];
         if (!uneven) {
           FxTileSrc3<F> src;
           src.t = &tile;
           src.base = base;
-          fx_eval3<F>(src, wx, wy, wz, R, G);
+          eval(src, R, G);
           fx_finish3<F>(R, G, emax, kp.inv_h, val, grad);
         } else {
           FxRawSrc3<F> src;
@@ -304,7 +311,7 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
           src.base = base;
           fine = src.scale();
           if (fine) {
-            fx_eval3<F>(src, wx, wy, wz, R, G);
+            eval(src, R, G);
             fx_finish3<F>(R, G, src.emax, kp.inv_h, val, grad);
             fine = src.fit();
           }
