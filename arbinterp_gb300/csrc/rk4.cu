@@ -23,29 +23,46 @@ __global__ void __launch_bounds__(256) norm_pairs_kernel(const float *g32, int64
   if (p < npts) pairs[p] = make_float2(__ldg(g32 + 4 * p + 3), __ldg(g32 + 4 * npts + p));
 }
 
-// Z-order key of each position over the interpolation box (10 bits per axis):
-// particles of one warp then gather neighbouring grid points.  Non-finite rows
-// sort last.  float32 is enough: the key orders the work, not the result.
+// Sort key of each position (30 bits): particles of one warp then gather
+// neighbouring grid points.  Non-finite rows sort last.  float32 is enough: the
+// key orders the work, not the result.
+// CELLS: 16-cell cubes in Z-order, inside a cube the x-rows of cells in Z-order
+// over (y, z), inside a row x.  A load costs one L1 wavefront per line that its
+// lanes touch, and a line is 16 points of one x-row: plain Z-order leaves 9.5
+// lines a load at 7 particles a cell.  Whole calls, Z-order against this: 2e5 x 25
+// steps on 128^3 1606 : 1350 us, 1e6 x 10 on 256^3 3364 : 2830.  A cloud that ends
+// just past a row of cubes has a few warps with one cell of every row, though,
+// and where an SM holds few warps the slowest one counts: 2e4 x 20 on 64^3 467 : 427
+// or 449 : 559 us, 4e4 516 : 646.  So Z-order over the box (10 bits an axis)
+// below CELLS_FROM particles.
+constexpr int64_t CELLS_FROM = 1 << 17;
 __device__ __forceinline__ uint32_t spread10(uint32_t v) {
   v = (v | v << 16) & 0x030000ffu;
   v = (v | v << 8) & 0x0300f00fu;
   v = (v | v << 4) & 0x030c30c3u;
   return (v | v << 2) & 0x09249249u;
 }
+__device__ __forceinline__ uint32_t spread4(uint32_t v) {
+  v = (v | v << 2) & 0x33u;
+  return (v | v << 1) & 0x55u;
+}
+template <bool CELLS>
 __global__ void __launch_bounds__(256) zorder_kernel(const double *state, int64_t n, double l0, double l1, double l2,
                                                      float s0, float s1, float s2, int32_t *keys) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double lo[3] = {l0, l1, l2};
   const float sc[3] = {s0, s1, s2};
-  uint32_t key = 0;
+  uint32_t c[3], key = 0;
   bool finite = true;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const float d = (float)(state[i * 6 + a] - lo[a]) * sc[a];
     finite &= fabsf(d) < 1e30f;
-    key |= spread10((uint32_t)fminf(fmaxf(d, 0.f), 1023.f)) << a;
+    c[a] = (uint32_t)fminf(fmaxf(d, 0.f), 1023.f);
+    key |= spread10(CELLS ? c[a] >> 4 : c[a]) << a;
   }
+  if (CELLS) key = key << 12 | (spread4(c[1] & 15) | spread4(c[2] & 15) << 1) << 4 | (c[0] & 15);
   keys[i] = finite ? (int32_t)key : 1 << 30;
 }
 
@@ -218,9 +235,17 @@ extern "C" int arb_norm_pairs(const arb_grid *g, float *pairs, arb_stream_t stre
 extern "C" int arb_zorder_keys(const arb_grid *g, const double *state, int64_t n, int32_t *keys, arb_stream_t stream) {
   if (!g || g->dim != 3 || n < 0 || (n > 0 && (!state || !keys))) return ARB_ERR_INVALID;
   if (n == 0) return ARB_OK;
+  const bool cells = n >= CELLS_FROM;
   float sc[3];
-  for (int a = 0; a < 3; ++a) sc[a] = (float)(1023.0 / (g->hi[a] - g->lo[a]));
-  zorder_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(state, n, g->lo[0], g->lo[1], g->lo[2],
-                                                                              sc[0], sc[1], sc[2], keys);
+  for (int a = 0; a < 3; ++a) {  // cells where an axis has at most 1023 of them, else 1023 steps
+    const double span = g->hi[a] - g->lo[a];
+    sc[a] = (float)(cells && span <= 1023.0 * g->h[a] ? 1.0 / g->h[a] : 1023.0 / span);
+  }
+  const unsigned b = (unsigned)((n + 255) / 256);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (cells)
+    zorder_kernel<true><<<b, 256, 0, s>>>(state, n, g->lo[0], g->lo[1], g->lo[2], sc[0], sc[1], sc[2], keys);
+  else
+    zorder_kernel<false><<<b, 256, 0, s>>>(state, n, g->lo[0], g->lo[1], g->lo[2], sc[0], sc[1], sc[2], keys);
   return launch_status();
 }

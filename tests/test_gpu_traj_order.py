@@ -8,7 +8,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 127, 128, 1000])
+@pytest.mark.parametrize("n", [1, 127, 128, 1000, (1 << 17) + 5])
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 @pytest.mark.parametrize("mode", ["scalar", "both"])
 def test_order_and_pairs_keep_the_bits(mode, prec, n):
