@@ -146,13 +146,20 @@ __host__ __device__ __forceinline__ int bank_class(int64_t cx, int64_t cy, int64
   return (int)((cx + 11 * cy + 9 * cz) & 15);
 }
 
-// 4D: the 8-byte bank slot (mod 16) of the cell's corner point in an unpadded
-// 7^4 tile of (hi, lo) pairs (x + 7 y + 49 z + 343 t, with 49 = 1 and
-// 343 = 7 mod 16).  Bin origins are multiples of 4, so the class from the
-// global cell coordinates is the local one plus a constant per bin: the
-// classes of one bin still map to 16 distinct slots.
+// 4D: the 8-byte bank slot (mod 16) of the cell's corner point in a 7^4 tile.
+// Mixed tiles have their z-planes 52 points apart and their t-slabs 364: x + 4 z
+// alone then takes every slot four times over a bin's cells, so the classes are
+// equally full (64 x 64 x 64 x 32, 1e7 queries, 305 a bin: 1815 -> 1665 us, 1.98 ->
+// 1.65 wavefronts an access in a model).  Unpadded, 49 = 1 and 343 = 7 mod 16, the
+// classes have 10 to 24 cells, and the crowded ones conflict at the end of every
+// bin; float64 tiles, bound by arithmetic, stay so (padded 1.5-3 % slower).  Bin
+// origins are multiples of 4, so the class from the global cell coordinates is
+// the local one plus a constant per bin: the classes of one bin still map to 16
+// distinct slots.
+constexpr int TILE4_Z = 52, TILE4_T = 364;
+template <bool PADDED>
 __host__ __device__ __forceinline__ int bank_class4(int64_t cx, int64_t cy, int64_t cz, int64_t ct) {
-  return (int)((cx + 7 * cy + cz + 7 * ct) & 15);
+  return (int)((cx + 7 * cy + (PADDED ? TILE4_Z : 1) * cz + (PADDED ? TILE4_T : 7) * ct) & 15);
 }
 
 // Float64 bins with enough queries to be staged (see launch_eval_fx).
@@ -247,7 +254,7 @@ __device__ __forceinline__ CoordStep bin_step(const arb_grid &g, const KParams &
       if constexpr (DIM == 3)
         b = (b << 4) | bank_class(c[0], c[1], c[2]);
       else
-        b = (b << 4) | bank_class4(c[0], c[1], c[2], c[3]);
+        b = (b << 4) | bank_class4<!EXACT>(c[0], c[1], c[2], c[3]);
     }
     bin = b;
   } else {
@@ -854,24 +861,31 @@ static bool launch_eval_binc(const arb_grid *g, const KParams &kp, const BinGeom
 // different 128-byte line per instruction and the kernel was L1-bound.
 // Bank order: an 8-byte shared load is served half-warp by half-warp, 16
 // slots of 8 bytes per wavefront, and point (i, j, k, l) of the block of a
-// cell of class c (bank_class4) lies in slot (c + i + 7 j + k + 7 l + const)
+// cell of class c (bank_class4) lies in slot (c + i + 7 j + 4 k + 12 l + const)
 // mod 16; placement writes each bin's queries round robin over its 16
 // classes, so in every level with all 16 classes a half-warp's 16 loads hit
 // 16 distinct slots: one wavefront, where 16 random queries need about three.
+// Bound by those wavefronts (82 % of its cycles before the tile was padded).
 constexpr int BIN4_EDGE = 4;
 constexpr int TILE4_EDGE = BIN4_EDGE + 3;
 constexpr int TILE4_PTS = TILE4_EDGE * TILE4_EDGE * TILE4_EDGE * TILE4_EDGE;
+constexpr int TILE4_SLOTS = (TILE4_EDGE - 1) * (TILE4_T + TILE4_Z + TILE4_EDGE + 1) + 1;
 constexpr int BIN4_THREADS = 128;
 
+// Slot of the corner point of a cell's block.
+__device__ __forceinline__ int tile4_base(const int64_t c[4], const int64_t o[4]) {
+  return (int)((c[3] - o[3]) * TILE4_T + (c[2] - o[2]) * TILE4_Z + (c[1] - o[1]) * TILE4_EDGE + (c[0] - o[0]));
+}
+
 struct BinTile4 {
-  float2 v[TILE4_PTS];  // [t][z][y][x] (hi, lo)
+  float2 v[TILE4_SLOTS];  // [t][z][y][x] (hi, lo)
 };
 
 struct TileBlock4 {  // a 4x4x4x4 block inside a staged tile
   const float2 *v;
   int base;  // tile index of the block corner
   __device__ __forceinline__ int at(int i, int j, int k, int l) const {
-    return base + ((l * TILE4_EDGE + k) * TILE4_EDGE + j) * TILE4_EDGE + i;
+    return base + l * TILE4_T + k * TILE4_Z + j * TILE4_EDGE + i;
   }
   template <int F>
   __device__ __forceinline__ void load(int p, int, float &hi, float &lo) const {
@@ -910,7 +924,8 @@ __device__ __forceinline__ void load_bin_tile4(const arb_grid &g, const BinGeom 
     const uint2 w = rows.row[r];
     const int ly = w.y & 0xff, lz = w.y >> 8 & 0xff, lt = w.y >> 16;
     if (!whole && (lx >= m[0] || ly >= m[1] || lz >= m[2] || lt >= m[3])) continue;
-    cp_async8(&t.v[e], g2 + lx + (narrow ? (int64_t)w.x : ((lt * nz + lz) * ny + ly) * nx));
+    cp_async8(&t.v[e + lz * (TILE4_Z - TILE4_EDGE * TILE4_EDGE) + lt * (TILE4_T - TILE4_EDGE * TILE4_EDGE * TILE4_EDGE)],
+              g2 + lx + (narrow ? (int64_t)w.x : ((lt * nz + lz) * ny + ly) * nx));
   }
 }
 
@@ -945,9 +960,7 @@ __global__ void __launch_bounds__(BIN4_THREADS, 4) eval_bin4_kernel(arb_grid g, 
         unpack_cell<4>(r.cell, c);
         TileBlock4 blk;
         blk.v = tiles[stage].v;
-        blk.base = (int)((((c[3] - og[3]) * TILE4_EDGE + (c[2] - og[2])) * TILE4_EDGE + (c[1] - og[1])) *
-                             TILE4_EDGE +
-                         (c[0] - og[0]));
+        blk.base = tile4_base(c, og);
         const float fr[4] = {r.f[0], r.f[1], r.f[2], r.f[3]};
         double val[1], grad[4];
         eval_otf4_mixed_block<1>(blk, kp, fr, val, grad);
