@@ -865,7 +865,7 @@ static bool launch_eval_binc(const arb_grid *g, const KParams &kp, const BinGeom
 // mod 16; placement writes each bin's queries round robin over its 16
 // classes, so in every level with all 16 classes a half-warp's 16 loads hit
 // 16 distinct slots: one wavefront, where 16 random queries need about three.
-// Bound by those wavefronts (82 % of its cycles before the tile was padded).
+// Bound by those wavefronts (77 % of its cycles; 82 % before the tile was padded).
 constexpr int BIN4_EDGE = 4;
 constexpr int TILE4_EDGE = BIN4_EDGE + 3;
 constexpr int TILE4_PTS = TILE4_EDGE * TILE4_EDGE * TILE4_EDGE * TILE4_EDGE;
