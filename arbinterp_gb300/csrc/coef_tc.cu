@@ -44,6 +44,7 @@
 
 #include "arb_common.cuh"
 #include "tc_ptx.cuh"
+#include "ws_ring.cuh"
 
 namespace arb {
 
@@ -409,6 +410,7 @@ constexpr int WS_THREADS = WS_PROD + WS_EPI + 64;
 constexpr int WS_TMEM_COLS = 512;                   // two accumulator stages of 3 x 64 columns
 constexpr uint32_t BAR_PROD = 1, BAR_EPI = 3;       // named barriers of the producer groups (1, 2) and the epilogue's (3, 4)
 constexpr int WS_FP = 3;                            // footprint buffers: boxes three tiles ahead
+using WsRing = FootprintRing<WS_FP, WS_PG>;
 
 template <int F>
 struct WsSmem {
@@ -419,7 +421,7 @@ struct WsSmem {
   int16_t hexp[4][2][TM];                  // scale exponents of half rows: [tile mod 4][half][row]
   float mrhi[4][TM], mrlo[4][TM];          // each row's corner value (hi, lo), by tile mod 4
   int mexp[4][TM];                         // each row's scale exponent
-  uint64_t fp_full[WS_FP], fp_empty[WS_FP], a_full[2], a_empty[2], acc_full[2], acc_empty[2];
+  uint64_t fp_full[WsRing::FULL], fp_empty[WS_FP], a_full[2], a_empty[2], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort;
 };
@@ -472,10 +474,8 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
     tc::tmem_relinquish();
   }
   if (tid == 0) {
-    for (int s = 0; s < WS_FP; ++s) {
-      tc::mbar_init(&sm.fp_full[s], 1);
-      tc::mbar_init(&sm.fp_empty[s], WS_GROUP / 32);
-    }
+    for (int s = 0; s < WsRing::FULL; ++s) tc::mbar_init(&sm.fp_full[s], 1);
+    for (int s = 0; s < WS_FP; ++s) tc::mbar_init(&sm.fp_empty[s], WS_GROUP / 32);
     for (int s = 0; s < 2; ++s) {
       tc::mbar_init(&sm.a_full[s], WS_GROUP / 32);
       tc::mbar_init(&sm.a_empty[s], 1);
@@ -505,9 +505,9 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
       const int64_t xr = tile / tpr;
       const int x0 = (int)((tile - xr * tpr) * S::C);
       const int cnt = tile - xr * tpr == tpr - 1 ? rem : S::C;
-      const int fs = k % WS_FP;
+      const int fs = WsRing::buffer(k);
       const bool live = (row & ~31) < cnt * F;           // some row of this warp is in the table
-      bool ok = !fail && ws_wait(sm, &sm.fp_full[fs], (uint32_t)(k / WS_FP) & 1u, WAIT_LIMIT, status);
+      bool ok = !fail && ws_wait(sm, &sm.fp_full[WsRing::full(k)], WsRing::full_parity(k), WAIT_LIMIT, status);
       float rhi = 0.f, rlo = 0.f, d[32], amax = 0.f;
 #pragma unroll
       for (int j = 0; j < 32; ++j) d[j] = 0.f;
@@ -650,17 +650,18 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
   } else if (warp == WS_WARP_FP && lane == 0) {
     // ---- footprint loader: boxes WS_FP tiles ahead ---------------------------
     auto issue_fp = [&](int k) {
-      const int s = k % WS_FP;
+      const int s = WsRing::buffer(k);
+      uint64_t *full = &sm.fp_full[WsRing::full(k)];
       const int64_t tile = tile_of(k);
       const int64_t xr = tile / tpr;
       const int x0 = (int)((tile - xr * tpr) * S::C);
       const int y = (int)(xr % ncy), z = (int)(xr / ncy);
-      tc::mbar_arrive_expect_tx(&sm.fp_full[s], (uint32_t)(S::HBYTES + S::LBYTES));
+      tc::mbar_arrive_expect_tx(full, (uint32_t)(S::HBYTES + S::LBYTES));
       if constexpr (F == 1) {
-        tc::tma_load_3d(sm.fp[s], &tmap_hi, x0 & ~1, y, z, &sm.fp_full[s]);
+        tc::tma_load_3d(sm.fp[s], &tmap_hi, x0 & ~1, y, z, full);
       } else {
-        tc::tma_load_3d(sm.fp[s], &tmap_hi, 4 * x0, y, z, &sm.fp_full[s]);
-        if constexpr (F == 4) tc::tma_load_3d(sm.fp[s] + S::HBYTES, &tmap_lo, x0 & ~3, y, z, &sm.fp_full[s]);
+        tc::tma_load_3d(sm.fp[s], &tmap_hi, 4 * x0, y, z, full);
+        if constexpr (F == 4) tc::tma_load_3d(sm.fp[s] + S::HBYTES, &tmap_lo, x0 & ~3, y, z, full);
       }
     };
     int fp_issued = 0;
@@ -668,13 +669,13 @@ __global__ void __launch_bounds__(WS_THREADS, 1) coef3_tma_kernel(const __grid_c
     // the footprint WS_FP tiles ahead, as soon as the producers have read
     // tile k's buffer (after their gather, long before its A tile is ready)
     for (int k = 0; k + WS_FP < nloc; ++k) {
-      if (!ws_wait(sm, &sm.fp_empty[k % WS_FP], (uint32_t)(k / WS_FP) & 1u, WAIT_LIMIT, status)) break;
+      if (!ws_wait(sm, &sm.fp_empty[WsRing::buffer(k)], WsRing::empty_parity(k), WAIT_LIMIT, status)) break;
       issue_fp(k + WS_FP);
       fp_issued = k + WS_FP + 1;
     }
     // no box load in flight when the CTA's shared memory is given back
     for (int kf = fp_issued - WS_FP > 0 ? fp_issued - WS_FP : 0; kf < fp_issued; ++kf)
-      (void)tc::mbar_wait_bounded(&sm.fp_full[kf % WS_FP], (uint32_t)(kf / WS_FP) & 1u, WAIT_LIMIT);
+      (void)tc::mbar_wait_bounded(&sm.fp_full[WsRing::full(kf)], WsRing::full_parity(kf), WAIT_LIMIT);
   } else if (warp == WS_WARP_MMA && lane == 0) {
     // ---- MMA issue -----------------------------------------------------------
     int mma_done = 0;
