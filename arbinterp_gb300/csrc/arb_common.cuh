@@ -124,8 +124,11 @@ struct FastAxis {
   int he;                             // biased exponent of h; 0 where axis_step_fx does not apply
 };
 
-// Range of the axis as keys, finite so that every NaN lies outside.
+// Range of the axis as keys, finite so that every NaN lies outside.  The keys tell
+// -0 from +0, float64 compares do not: a bound at zero takes in both.
 __host__ __device__ __forceinline__ void fast_axis_range(FastAxis &f, unsigned long long lo, unsigned long long hi) {
+  if (lo == 0) lo = 0x8000000000000000ULL;
+  if (hi == 0x8000000000000000ULL) hi = 0;
   const unsigned long long ninf = ord_key_bits(0xfff0000000000000ULL), pinf = ord_key_bits(0x7ff0000000000000ULL);
   f.lo_key = ord_key_bits(lo) > ninf ? ord_key_bits(lo) : ninf;
   f.hi_key = ord_key_bits(hi) < pinf ? ord_key_bits(hi) : pinf;
