@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
     }
   }
   // records that need no evaluation (out of volume, NaN, sentinel column)
-  for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
+  for (int64_t t = items.special(bg, nq) + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
        t += (int64_t)gridDim.x * blockDim.x) {
     const QRec64<3> q = recs[t];
     write_const<3, F>(o, q.row, rec64_cell<3>(q) != NAN_CELL<3> && !g.sentinel_nan ? 0.0 : qnan());
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(FX_THREADS, 2) eval_fx4_kernel(arb_grid g, KPa
     }
     __syncthreads();
   }
-  for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
+  for (int64_t t = items.special(bg, nq) + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
        t += (int64_t)gridDim.x * blockDim.x) {
     const QRec64<4> q = recs[t];
     write_const<4, F>(o, q.row, rec64_cell<4>(q) != NAN_CELL<4> && !g.sentinel_nan ? 0.0 : qnan());

@@ -211,11 +211,13 @@ static size_t carve(SortedWork *w, void *base, const arb_grid *g, int precision,
     return r;
   };
   SortedWork t;
+  // the records and the histogram's first word lie where every layout of these
+  // rows has them (BinGeom::cls depends on the field count and the bin shift)
+  t.rec = take((mixed ? sizeof(QRec) : g->dim == 3 ? sizeof(QRec64<3>) : sizeof(QRec64<4>)) * nq);
   t.hist = (uint32_t *)take(sizeof(uint32_t) * (bg.nsub + 1));
   t.offs = (uint32_t *)take(sizeof(uint32_t) * (bg.nsub + 1));
   t.part = (uint32_t *)take(sizeof(uint32_t) * scan_blocks(bg.nsub + 1));
   t.hdr = bg.cls ? (BinHdr *)take(sizeof(BinHdr) * bg.nbins) : nullptr;
-  t.rec = take((mixed ? sizeof(QRec) : g->dim == 3 ? sizeof(QRec64<3>) : sizeof(QRec64<4>)) * nq);
   if (w) *w = t;
   if (mixed) return off;
   // The stated need of a float64 call is 48 bytes a row and one counter pair a
@@ -504,10 +506,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const uint32_t
 // records is cut: its first share is the bin's own item, each further one an
 // item (bin, share number) in the list that split_kernel leaves in the
 // histogram (which placement has counted down to zero; word 0 is the list's
-// length).  split_share bounds the list by the room there.
-struct BinItem {
-  uint32_t bin, part;
-};
+// length, and its bit CLASSED says that the records lie in bins with bank
+// classes).  split_share bounds the list by the room there.
+constexpr uint32_t CLASSED = 0x80000000u;
 
 // About four items for each of ~600 resident CTAs.  Where the bins alone make
 // two, only a bin of twice the mean is cut (its tile is staged again for every
@@ -523,15 +524,18 @@ static inline uint32_t split_share(const BinGeom &bg, int64_t nq) {
 __global__ void __launch_bounds__(256) split_kernel(const uint32_t *offs, BinGeom bg, uint32_t share, uint32_t *hist) {
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b >= bg.nbins) return;
+  if (b == 0) atomicOr(hist, CLASSED);
   const uint32_t n = offs[(b + 1) << bg.cls] - offs[b << bg.cls];
   if (n <= share) return;
-  const uint32_t more = (n - 1) / share, at = atomicAdd(hist, more);
+  const uint32_t more = (n - 1) / share, at = atomicAdd(hist, more) & ~CLASSED;
   for (uint32_t p = 0; p < more; ++p)
     reinterpret_cast<uint2 *>(hist + 2)[at + p] = make_uint2((uint32_t)b, p + 1);
 }
 
 // The items of a staged kernel: the further shares first (each a full one or
-// the rest of a crowded bin), then every bin's own.
+// the rest of a crowded bin), then every bin's own.  None where the records came
+// without classes, binned by a descriptor of another field count or bin shift:
+// eval_unclassed_kernel takes those.
 struct BinItems {
   const uint32_t *offs;
   const uint2 *more;
@@ -539,8 +543,15 @@ struct BinItems {
   uint32_t share;
   int cls;
   __device__ __forceinline__ BinItems(const SortedWork &w, const BinGeom &bg, uint32_t share_)
-      : offs(w.offs), more(reinterpret_cast<const uint2 *>(w.hist + 2)), nmore(w.hist[0]), n(nmore + bg.nbins),
-        share(share_), cls(bg.cls) {}
+      : offs(w.offs), more(reinterpret_cast<const uint2 *>(w.hist + 2)), share(share_), cls(bg.cls) {
+    const uint32_t head = w.hist[0];
+    nmore = head & ~CLASSED;
+    n = head & CLASSED ? nmore + bg.nbins : 0;
+  }
+  // First record that needs no evaluation (of nq).
+  __device__ __forceinline__ int64_t special(const BinGeom &bg, int64_t nq) const {
+    return n ? (int64_t)offs[bg.nsub] : nq;
+  }
   // Bin of item i and its records [t0, t1); t0 == t1 past the end.
   __device__ __forceinline__ int64_t get(int64_t i, uint32_t &t0, uint32_t &t1) const {
     t0 = t1 = 0;
@@ -559,12 +570,9 @@ struct BinItems {
 };
 
 template <int DIM, int F, bool MIXED, bool TABLE>
-__global__ void __launch_bounds__(DIM == 3 ? 256 : 128, MIXED ? 0 : (DIM == 3 || F == 4 ? 2 : 3)) eval_sorted_kernel(arb_grid g, KParams kp,
-                                                                           int64_t nq, arb_query_out o,
-                                                                           SortedWork w) {
+__device__ __forceinline__ void eval_record(const arb_grid &g, const KParams &kp, int64_t t, const arb_query_out &o,
+                                            const SortedWork &w) {
   using T = typename std::conditional<MIXED, float, double>::type;
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nq) return;
   int64_t i, c[DIM];
   T fr[DIM];
   bool sentinel;
@@ -583,6 +591,25 @@ __global__ void __launch_bounds__(DIM == 3 ? 256 : 128, MIXED ? 0 : (DIM == 3 ||
     eval_otf4<F, MIXED>(g, kp, c, fr, val, grad);
   }
   write_vals<DIM, F>(o, i, val, grad);
+}
+
+template <int DIM, int F, bool MIXED, bool TABLE>
+__global__ void __launch_bounds__(DIM == 3 ? 256 : 128, MIXED ? 0 : (DIM == 3 || F == 4 ? 2 : 3)) eval_sorted_kernel(arb_grid g, KParams kp,
+                                                                           int64_t nq, arb_query_out o,
+                                                                           SortedWork w) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t < nq) eval_record<DIM, F, MIXED, TABLE>(g, kp, t, o, w);
+}
+
+// The same where a staged kernel found records without bank classes; nothing
+// otherwise.  Launched behind the staged kernel by the call that evaluates
+// records which another descriptor may have binned.
+template <int DIM, int F, bool MIXED>
+__global__ void __launch_bounds__(DIM == 3 ? 256 : 128, MIXED ? 0 : (DIM == 3 || F == 4 ? 2 : 3))
+    eval_unclassed_kernel(arb_grid g, KParams kp, int64_t nq, arb_query_out o, SortedWork w) {
+  if (w.hist[0] & CLASSED) return;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq; t += (int64_t)gridDim.x * blockDim.x)
+    eval_record<DIM, F, MIXED, false>(g, kp, t, o, w);
 }
 
 // ---- bin-staged evaluation (3D, mixed, 8^3-cell bins) -------------------------
@@ -806,7 +833,7 @@ __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) e
     for (int a = 0; a < 3; ++a) og[a] = on[a];
   }
   // records that need no evaluation (out of volume, NaN, sentinel column)
-  for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
+  for (int64_t t = items.special(bg, nq) + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
        t += (int64_t)gridDim.x * blockDim.x) {
     const QRec r = recs[t];
     write_const<3, F>(o, r.row, (r.cell & 1ULL) && !g.sentinel_nan ? 0.0 : qnan());
@@ -974,7 +1001,7 @@ __global__ void __launch_bounds__(BIN4_THREADS, 4) eval_bin4_kernel(arb_grid g, 
     t1 = n1;
   }
   // records that need no evaluation (out of volume, NaN, sentinel column)
-  for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
+  for (int64_t t = items.special(bg, nq) + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
        t += (int64_t)gridDim.x * blockDim.x) {
     const QRec r = recs[t];
     write_const<4, 1>(o, r.row, (r.cell & 1ULL) && !g.sentinel_nan ? 0.0 : qnan());
@@ -1131,14 +1158,33 @@ __global__ void __launch_bounds__(256) eval_tab_coop_kernel(arb_grid g, KParams 
   }
 }
 
+// own: the records were binned by this call, with this descriptor.
 template <int DIM, bool MIXED>
 static void launch_eval(const arb_grid *g, const KParams &kp, int64_t nq, const arb_query_out *out,
-                        const SortedWork &w, bool table, cudaStream_t s) {
+                        const SortedWork &w, bool table, bool own, cudaStream_t s) {
   const BinGeom bg = bin_geom(g, MIXED ? ARB_PREC_MIXED : ARB_PREC_FP64, nq);
-  if (DIM == 3 && MIXED && !table && launch_eval_binc(g, kp, bg, nq, out, w, s)) return;
-  if (DIM == 4 && MIXED && !table && launch_eval_bin4(g, kp, bg, nq, out, w, s)) return;
-  if (!MIXED && !table && launch_eval_fx<DIM>(g, kp, bg, nq, out, w, s)) return;
   const int TE = DIM == 3 ? 256 : 128;
+  bool staged = false;
+  if (!table) {
+    if constexpr (!MIXED)
+      staged = launch_eval_fx<DIM>(g, kp, bg, nq, out, w, s);
+    else if constexpr (DIM == 3)
+      staged = launch_eval_binc(g, kp, bg, nq, out, w, s);
+    else
+      staged = launch_eval_bin4(g, kp, bg, nq, out, w, s);
+  }
+  if (staged) {
+    if (own) return;
+    const unsigned BU = (unsigned)min((nq + TE - 1) / TE, (int64_t)device_sms() * 16);
+#define EU(FF) eval_unclassed_kernel<DIM, FF, MIXED><<<BU, TE, 0, s>>>(*g, kp, nq, *out, w)
+    if constexpr (DIM == 4 && MIXED) {
+      EU(1);  // the staged field count
+    } else {
+      switch (g->nfield) { case 1: EU(1); break; case 3: EU(3); break; default: EU(4); break; }
+    }
+#undef EU
+    return;
+  }
   const unsigned BE = (unsigned)((nq + TE - 1) / TE);
 #define ES(FF, TAB) eval_sorted_kernel<DIM, FF, MIXED, TAB><<<BE, TE, 0, s>>>(*g, kp, nq, *out, w)
   if (table) {
@@ -1319,7 +1365,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) adjoint_bin_kernel(arb_grid g, KP
   }
   // rows outside the volume, NaN rows and the sentinel column: no gradient
   if (q_grad)
-    for (int64_t t = (int64_t)w.offs[bg.nsub] + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
+    for (int64_t t = items.special(bg, nq) + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nq;
          t += (int64_t)gridDim.x * blockDim.x) {
       const int64_t row = recs[t].row;
       q_grad[row * 3] = q_grad[row * 3 + 1] = q_grad[row * 3 + 2] = 0.0;
@@ -1422,18 +1468,18 @@ extern "C" int arb_query_eval_sorted(const arb_grid *g, int32_t precision, int32
   if (g->dim == 3) {
     if (mixed) {
       launch_bin<3, true>(g, kp, bg, q, nq, q_stride, q_writeback, out, status, w, s);
-      launch_eval<3, true>(g, kp, nq, out, w, use_table, s);
+      launch_eval<3, true>(g, kp, nq, out, w, use_table, true, s);
     } else {
       launch_bin<3, false>(g, kp, bg, q, nq, q_stride, q_writeback, out, status, w, s);
-      launch_eval<3, false>(g, kp, nq, out, w, use_table, s);
+      launch_eval<3, false>(g, kp, nq, out, w, use_table, true, s);
     }
   } else {
     if (mixed) {
       launch_bin<4, true>(g, kp, bg, q, nq, q_stride, q_writeback, out, status, w, s);
-      launch_eval<4, true>(g, kp, nq, out, w, use_table, s);
+      launch_eval<4, true>(g, kp, nq, out, w, use_table, true, s);
     } else {
       launch_bin<4, false>(g, kp, bg, q, nq, q_stride, q_writeback, out, status, w, s);
-      launch_eval<4, false>(g, kp, nq, out, w, use_table, s);
+      launch_eval<4, false>(g, kp, nq, out, w, use_table, true, s);
     }
   }
   return launch_status();
@@ -1441,7 +1487,7 @@ extern "C" int arb_query_eval_sorted(const arb_grid *g, int32_t precision, int32
 
 // Binning only: the first half of arb_query_eval_sorted.  The workspace then
 // holds the bin-ordered records, which depend on the query points and the
-// grid geometry but not on the field values.
+// axes but not on the fields.
 extern "C" int arb_query_bin(const arb_grid *g, int32_t precision, double *q, int64_t nq, int64_t q_stride,
                              int32_t q_writeback, const arb_query_out *out, void *work, size_t work_bytes,
                              int32_t *status, arb_stream_t stream) {
@@ -1474,7 +1520,7 @@ extern "C" int arb_query_bin(const arb_grid *g, int32_t precision, double *q, in
 }
 
 // Evaluation only, from a workspace filled by arb_query_bin for the same
-// query rows and a grid of the same geometry (values may differ).
+// query rows, precision and axes (values, field count and bin shift may differ).
 extern "C" int arb_query_eval_binned(const arb_grid *g, int32_t precision, int32_t use_table, int64_t nq,
                                      const arb_query_out *out, void *work, size_t work_bytes,
                                      arb_stream_t stream) {
@@ -1494,11 +1540,11 @@ extern "C" int arb_query_eval_binned(const arb_grid *g, int32_t precision, int32
   out = &out_norm;
   const KParams kp = make_kparams(g);
   if (g->dim == 3) {
-    if (mixed) launch_eval<3, true>(g, kp, nq, out, w, use_table, s);
-    else launch_eval<3, false>(g, kp, nq, out, w, use_table, s);
+    if (mixed) launch_eval<3, true>(g, kp, nq, out, w, use_table, false, s);
+    else launch_eval<3, false>(g, kp, nq, out, w, use_table, false, s);
   } else {
-    if (mixed) launch_eval<4, true>(g, kp, nq, out, w, use_table, s);
-    else launch_eval<4, false>(g, kp, nq, out, w, use_table, s);
+    if (mixed) launch_eval<4, true>(g, kp, nq, out, w, use_table, false, s);
+    else launch_eval<4, false>(g, kp, nq, out, w, use_table, false, s);
   }
   return launch_status();
 }

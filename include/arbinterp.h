@@ -294,9 +294,13 @@ int arb_batched_launch(const arb_grid *grids, int32_t nfields, int32_t nfield, c
  *      arb_query_bin: index step, out-of-volume bookkeeping (inds, oob rows,
  *      q write-back, status) and the bin-ordered records in `work`.
  *      arb_query_eval_binned: evaluation from those records into
- *      out->comps/norms/grads.  The records depend on the query points and
- *      the grid geometry only, so the same points can be re-evaluated after
- *      the field values change (same geometry) without binning again. */
+ *      out->comps/norms/grads.  The records depend on the query points, the
+ *      precision and the axes (n, lo, hi, h) only, so the same points can be
+ *      evaluated on other values and other fields of the same axes without
+ *      binning again: nfield, kind and bin_shift may differ between the two
+ *      calls (records grouped otherwise than a descriptor's own kernel wants
+ *      them are evaluated one lane a query).  work_bytes: at least what
+ *      arb_query_sorted_work_bytes gives for each of the descriptors. */
 int arb_query_bin(const arb_grid *g, int32_t precision, double *q, int64_t nq, int64_t q_stride,
                   int32_t q_writeback, const arb_query_out *out, void *work, size_t work_bytes,
                   int32_t *status, arb_stream_t stream);
