@@ -326,6 +326,27 @@ __device__ __forceinline__ int64_t flat_step(const int32_t fl[4], const arb_grid
   return (int64_t)idx;
 }
 
+// Floors that 32 bits do not hold (an axis whose first spacing is tiny): the
+// floor saturates, past every cell of its axis, and the index is formed from the
+// 64-bit floors, saturated far past every table.
+__device__ __forceinline__ int32_t narrow_floor(int64_t k) {
+  return (unsigned long long)k > 0x7fffffffULL ? 0x7fffffff : (int32_t)k;
+}
+template <int DIM>
+struct WideSteps {
+  int64_t k[DIM], m[DIM];  // floors, cells per axis
+};
+template <int DIM>
+static __device__ __noinline__ int64_t wide_index(WideSteps<DIM> w) {
+  unsigned long long idx = 0;
+#pragma unroll 1
+  for (int a = DIM - 1; a >= 0; --a) {
+    const unsigned __int128 v = (unsigned __int128)idx * (unsigned long long)w.m[a] + (unsigned long long)w.k[a];
+    idx = v > (1ULL << 62) ? 1ULL << 62 : (unsigned long long)v;
+  }
+  return (int64_t)idx;
+}
+
 struct AxisStep64 {
   double k, frac;
 };
@@ -366,13 +387,24 @@ __device__ __forceinline__ CoordStep coord_step_fx(const double *qrow, const Fas
     return s;
   }
   if (slow) {
+    WideSteps<DIM> w;
+    bool wide = false;
 #pragma unroll
-    for (int a = 0; a < DIM; ++a)
+    for (int a = 0; a < DIM; ++a) {
+      w.k[a] = s.fl[a];
+      w.m[a] = g.n[a] - 3;
       if (!fine[a]) {
         const AxisStep64 r = axis_step_div(__dsub_rn(qrow[a], ax[a].lo), ax[a].h);
-        s.fl[a] = (int32_t)r.k;
+        w.k[a] = (int64_t)r.k;
+        s.fl[a] = narrow_floor(w.k[a]);
         frac[a] = r.frac;
       }
+      wide |= s.fl[a] != w.k[a];
+    }
+    if (wide) {
+      s.idx = wide_index<DIM>(w);
+      return s;
+    }
   }
   s.idx = flat_step<DIM>(s.fl, g);
   return s;
@@ -447,13 +479,24 @@ __device__ __forceinline__ CoordStep coord_step_fast(const double *qrow, const F
     return s;
   }
   if (slow) {
+    WideSteps<DIM> w;
+    bool wide = false;
 #pragma unroll
-    for (int a = 0; a < DIM; ++a)
+    for (int a = 0; a < DIM; ++a) {
+      w.k[a] = s.fl[a];
+      w.m[a] = g.n[a] - 3;
       if (!fine[a]) {
         const AxisStep r = axis_step_rest(qrow[a], ax[a]);
-        s.fl[a] = (int32_t)r.k;
+        w.k[a] = r.k;
+        s.fl[a] = narrow_floor(w.k[a]);
         frac[a] = r.fr;
       }
+      wide |= s.fl[a] != w.k[a];
+    }
+    if (wide) {
+      s.idx = wide_index<DIM>(w);
+      return s;
+    }
   }
   s.idx = flat_step<DIM>(s.fl, g);
   return s;
