@@ -28,6 +28,7 @@
 
 #include <mutex>
 
+#include "bin_shares.cuh"
 #include "eval.cuh"
 
 namespace arb {
@@ -501,33 +502,22 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const uint32_t
 }
 
 // ---- shares of crowded bins ----------------------------------------------------
-// A staged kernel takes one bin per CTA.  Clouds crowd a few bins, and small
-// grids have fewer bins than the GPU has CTAs, so a bin of more than `share`
-// records is cut: its first share is the bin's own item, each further one an
-// item (bin, share number) in the list that split_kernel leaves in the
+// A bin of more than bin_share() records is cut (bin_shares.cuh): its first share
+// is the bin's own item, each further one an item (bin, share number) in the
+// list that split_kernel leaves in the
 // histogram (which placement has counted down to zero; word 0 is the list's
 // length, and its bit CLASSED says that the records lie in bins with bank
-// classes).  split_share bounds the list by the room there.
+// classes).  bin_share bounds the list by the room there.
 constexpr uint32_t CLASSED = 0x80000000u;
-
-// About four items for each of ~600 resident CTAs.  Where the bins alone make
-// two, only a bin of twice the mean is cut (its tile is staged again for every
-// share: cutting 1220-record bins at 512 cost 10 %).  At least 512, and nq / 6 a
-// bin at most, for the list's room.
-static inline uint32_t split_share(const BinGeom &bg, int64_t nq) {
-  int64_t s = nq / 2432;
-  if (bg.nbins >= 1216 && s < 2 * nq / bg.nbins) s = 2 * nq / bg.nbins;
-  if (s < nq / (6 * bg.nbins)) s = nq / (6 * bg.nbins);
-  return (uint32_t)(s + 1 > 512 ? s + 1 : 512);
-}
 
 __global__ void __launch_bounds__(256) split_kernel(const uint32_t *offs, BinGeom bg, uint32_t share, uint32_t *hist) {
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b >= bg.nbins) return;
   if (b == 0) atomicOr(hist, CLASSED);
   const uint32_t n = offs[(b + 1) << bg.cls] - offs[b << bg.cls];
-  if (n <= share) return;
-  const uint32_t more = (n - 1) / share, at = atomicAdd(hist, more) & ~CLASSED;
+  const uint32_t more = bin_more_shares(n, share);
+  if (!more) return;
+  const uint32_t at = atomicAdd(hist, more) & ~CLASSED;
   for (uint32_t p = 0; p < more; ++p)
     reinterpret_cast<uint2 *>(hist + 2)[at + p] = make_uint2((uint32_t)b, p + 1);
 }
@@ -563,8 +553,8 @@ struct BinItems {
       b = m.x;
       part = m.y;
     }
-    t0 = offs[b << cls] + part * share;
-    t1 = min(offs[(b + 1) << cls], t0 + share);
+    t0 = bin_first(offs[b << cls], part, share);
+    t1 = bin_end(t0, offs[(b + 1) << cls], share);
     return b;
   }
 };
@@ -799,10 +789,10 @@ __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) e
     if (t1 > t0) {
       // the next record is loaded while this one is evaluated
       QRec rnext;
-      if (t0 + threadIdx.x < t1) rnext = recs[t0 + threadIdx.x];
-      for (uint32_t t = t0 + threadIdx.x; t < t1; t += BINC_THREADS) {
+      if (threadIdx.x < t1 - t0) rnext = recs[t0 + threadIdx.x];
+      for (uint32_t t = t0 + threadIdx.x; t - t0 < t1 - t0; t += BINC_THREADS) {
         const QRec r = rnext;
-        if (t + BINC_THREADS < t1) rnext = recs[t + BINC_THREADS];
+        if (t + BINC_THREADS - t0 < t1 - t0) rnext = recs[t + BINC_THREADS];
         int64_t c[3];
         unpack_cell<3>(r.cell, c);
         const int bi = (((int)c[2] - og[2]) * TILE_EDGE + ((int)c[1] - og[1])) * TILE_EDGE + ((int)c[0] - og[0]);
@@ -863,7 +853,7 @@ static bool launch_eval_binc_f(const arb_grid *g, const KParams &kp, const BinGe
     per_sm[dev] = n;
   }
   int64_t grid = (int64_t)sm_count_sorted() * per_sm[dev];
-  const uint32_t share = split_share(bg, nq);
+  const uint32_t share = bin_share(bg.nbins, nq);
   const int64_t items = bg.nbins + nq / share;  // at most
   if (grid > items) grid = items;
   eval_binc_kernel<F><<<(unsigned)grid, BINC_THREADS, smem, s>>>(*g, kp, bg, nq, *out, w, share);
@@ -981,7 +971,7 @@ __global__ void __launch_bounds__(BIN4_THREADS, 4) eval_bin4_kernel(arb_grid g, 
     if (t1 > t0) {
       int64_t og[4];
       bin_origin4(b, bg, og);
-      for (uint32_t t = t0 + threadIdx.x; t < t1; t += BIN4_THREADS) {
+      for (uint32_t t = t0 + threadIdx.x; t - t0 < t1 - t0; t += BIN4_THREADS) {
         const QRec r = recs[t];
         int64_t c[4];
         unpack_cell<4>(r.cell, c);
@@ -1028,7 +1018,7 @@ static bool launch_eval_bin4(const arb_grid *g, const KParams &kp, const BinGeom
     per_sm[dev] = n;
   }
   int64_t grid = (int64_t)sm_count_sorted() * per_sm[dev];
-  const uint32_t share = split_share(bg, nq);
+  const uint32_t share = bin_share(bg.nbins, nq);
   const int64_t items = bg.nbins + nq / share;  // at most
   if (grid > items) grid = items;
   eval_bin4_kernel<<<(unsigned)grid, BIN4_THREADS, smem, s>>>(*g, kp, bg, nq, *out, w, share);
@@ -1052,7 +1042,7 @@ static void launch_bin(const arb_grid *g, const KParams &kp, const BinGeom &bg, 
   if (nb > 1) scan_part_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(w.hist, nh, w.part);
   scan_apply_kernel<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(w.hist, nh, w.part, w.offs, w.hdr, bg.nbins);
   bin_place_kernel<DIM, !MIXED, T><<<B, TB, 0, s>>>(*g, kp, bg, q, nq, qs, w);
-  if (bg.cls) split_kernel<<<(unsigned)((bg.nbins + 255) / 256), 256, 0, s>>>(w.offs, bg, split_share(bg, nq), w.hist);
+  if (bg.cls) split_kernel<<<(unsigned)((bg.nbins + 255) / 256), 256, 0, s>>>(w.offs, bg, bin_share(bg.nbins, nq), w.hist);
 }
 
 // Table evaluation, 8 lanes per query.  A cell's block is F fields x R rows
@@ -1252,9 +1242,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) adjoint_bin_kernel(arb_grid g, KP
     __syncthreads();
     if (t1 > t0) {
       const float2 *tv = tiles[stage].v;
-      for (uint32_t tw = t0 + threadIdx.x / 32 * 32; tw < t1; tw += ADJ_THREADS) {  // warps stay whole
+      for (uint32_t tw = t0 + threadIdx.x / 32 * 32; tw - t0 < t1 - t0; tw += ADJ_THREADS) {  // warps stay whole
         const uint32_t t = tw + (threadIdx.x & 31);
-        bool on = t < t1;
+        bool on = t - t0 < t1 - t0;
         const QRec r = recs[on ? t : t0];
         const int64_t row = r.row;
         const float dv = on && dval ? (float)dval[row] : 0.f;
@@ -1613,7 +1603,7 @@ extern "C" int arb_adjoint_binned(const arb_grid *g, int32_t precision, const do
     per_sm[dev] = n;
   }
   int64_t grid = (int64_t)sm_count_sorted() * per_sm[dev];
-  const uint32_t share = split_share(bg, nq);
+  const uint32_t share = bin_share(bg.nbins, nq);
   const int64_t items = bg.nbins + nq / share;  // at most
   if (grid > items) grid = items;
   adjoint_bin_kernel<<<(unsigned)grid, ADJ_THREADS, smem, s>>>(gb, kp, bg, nq, dval, dgrad, (float *)grid_grad,
