@@ -597,8 +597,23 @@ static __device__ __noinline__ EvalOut<F, 3> eval_otf3_f64(const double *grid, i
   return o;
 }
 
+// A query on a grid point (all fractions zero).  Its value is the sample and its
+// derivatives are central differences, each rounded once, as float64 arithmetic
+// gives them; in the block's scale a sample below 2^-8 of the largest would lose bits.
+template <int N>
+__device__ __forceinline__ bool at_node(const double frac[N]) {
+  unsigned long long b = 0;
+#pragma unroll
+  for (int a = 0; a < N; ++a) b |= (unsigned long long)__double_as_longlong(frac[a]);
+  return b == 0;
+}
+__device__ __forceinline__ double node_slope(const double *p, int64_t step, double inv_h) {
+  return (0.5 * __ldg(p + step) - 0.5 * __ldg(p - step)) * inv_h;
+}
+
 // The block as a whole sets the scale: blocks with a sample far above the
-// query's own cell, or float64 arithmetic where the scaling does not hold.
+// query's own cell; or float64 arithmetic where the scaling does not hold; or a
+// grid point, whose block is all finite.
 template <int F, int STEP>
 static __device__ __noinline__ EvalOut<F, 3> eval_otf3_full(const double *grid, int64_t nx, int64_t ny, EvalArgs<3> in) {
   FxGrid3<F, STEP> src;
@@ -606,6 +621,16 @@ static __device__ __noinline__ EvalOut<F, 3> eval_otf3_full(const double *grid, 
   src.sy = nx * STEP;
   src.sz = nx * ny * STEP;
   if (!src.template scale<true>()) return eval_otf3_f64<F, STEP>(grid, nx, ny, in);
+  if (at_node<3>(in.frac)) {
+    const double *p = src.at(1, 1, 1);
+    EvalOut<F, 3> o;
+#pragma unroll
+    for (int f = 0; f < F; ++f) o.val[f] = __ldg(p + f);
+    o.grad[0] = node_slope(p + F - 1, STEP, in.inv_h[0]);
+    o.grad[1] = node_slope(p + F - 1, src.sy, in.inv_h[1]);
+    o.grad[2] = node_slope(p + F - 1, src.sz, in.inv_h[2]);
+    return o;
+  }
   FxW wx, wy, wz;
   fx_axis<1>(fx_bits(in.frac[0]), wx);
   fx_axis<1>(fx_bits(in.frac[1]), wy);
@@ -650,7 +675,7 @@ __device__ __forceinline__ void eval_otf3_fx(const arb_grid &g, const KParams &k
   src.p = g.grid64 + ((c[2] * ny + c[1]) * nx + c[0]) * STEP + (STEP - F);
   src.sy = nx * STEP;
   src.sz = nx * ny * STEP;
-  bool ok = src.template scale<false>();
+  bool ok = !at_node<3>(frac) && src.template scale<false>();
   if (ok) {
     FxW wx, wy, wz;
     fx_axis<1>(fx_bits(frac[0]), wx);
@@ -1041,6 +1066,16 @@ static __device__ __noinline__ EvalOut<1, 4> eval_otf4_full(Grid4Ref r, EvalArgs
   FxGrid4 src;
   r.block(src, in.c);
   if (!src.scale<true>()) return eval_otf4_f64(r.grid, r.nx, r.ny, r.nz, r.F, r.f, GRADF, in);
+  if (at_node<4>(in.frac)) {
+    const double *p = src.at(1, 1, 1, 1);
+    EvalOut<1, 4> o;
+    o.val[0] = __ldg(p);
+    o.grad[0] = GRADF ? node_slope(p, src.step, in.inv_h[0]) : 0.0;
+    o.grad[1] = GRADF ? node_slope(p, src.sy, in.inv_h[1]) : 0.0;
+    o.grad[2] = GRADF ? node_slope(p, src.sz, in.inv_h[2]) : 0.0;
+    o.grad[3] = GRADF ? node_slope(p, src.st, in.inv_h[3]) : 0.0;
+    return o;
+  }
   FxW w[2];
   fx_weights4(in.frac, w);
   long long R, G[4];
@@ -1076,7 +1111,7 @@ __device__ __forceinline__ void eval_otf4_fx(const arb_grid &g, const KParams &k
                                              const FxW w[2], const double frac[4], double &val, double grad[4]) {
   FxGrid4 src;
   Grid4Ref{g.grid64, g.n[0], g.n[1], g.n[2], F, f}.block(src, c);
-  bool ok = src.scale<false>();
+  bool ok = !at_node<4>(frac) && src.scale<false>();
   if (ok) {
     long long R, G[4];
     fx_eval4<GRADF>(src, w, FxZT(), R, G);

@@ -284,8 +284,8 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
       const double fr[3] = {rec64_frac<3>(q, 0), rec64_frac<3>(q, 1), rec64_frac<3>(q, 2)};
       double val[F], grad[3] = {0.0, 0.0, 0.0};
       const int base = (((int)c[2] - og[2]) * TILE_EDGE + ((int)c[1] - og[1])) * TILE_EDGE + ((int)c[0] - og[0]);
-      bool fine = ok;
-      if (ok) {
+      bool fine = ok && !at_node<3>(fr);
+      if (fine) {
         FxW wx, wy, wz;
         fx_axis<1>(fx_bits(fr[0]), wx);
         fx_axis<1>(fx_bits(fr[1]), wy);
@@ -466,6 +466,7 @@ __global__ void __launch_bounds__(FX_THREADS, 2) eval_fx4_kernel(arb_grid g, KPa
       cell_coords<4>((int64_t)rec64_cell<4>(q), g, c);
       const double fr[4] = {rec64_frac<4>(q, 0), rec64_frac<4>(q, 1), rec64_frac<4>(q, 2), rec64_frac<4>(q, 3)};
       double val[F], grad[4] = {0.0, 0.0, 0.0, 0.0};
+      const bool node = at_node<4>(fr);
       FxW wt[2];
       fx_weights4(fr, wt);
       const int base = (int)((((c[3] - og[3]) * TILE4_EDGE + (c[2] - og[2])) * TILE4_EDGE + (c[1] - og[1])) * TILE4_EDGE +
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(FX_THREADS, 2) eval_fx4_kernel(arb_grid g, KPa
       // field f in the tile's scale or its own; false: neither holds it
       auto contract = [&](auto gradf, int f, double &v, double gr[4]) {
         constexpr bool GRADF = decltype(gradf)::value;
-        if (!ok) return false;
+        if (!ok || node) return false;
         long long R, G[4];
         int e = emax[0];
         bool fine = true;
