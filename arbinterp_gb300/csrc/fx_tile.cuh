@@ -112,7 +112,7 @@ struct FxRawSrc3 {
   __device__ __forceinline__ bool fit() const {
     bool ok = true;
 #pragma unroll
-    for (int f = 0; f < F; ++f) ok &= (int)((over[f] + 1) >> 20) <= emax[f];
+    for (int f = 0; f < F; ++f) ok &= fx_fits(over[f], emax[f]);
     return ok;
   }
   __device__ __forceinline__ bool scale() {
@@ -131,9 +131,7 @@ struct FxRawSrc3 {
     bool ok = true;
 #pragma unroll
     for (int f = 0; f < F; ++f) {
-      ok &= m[f].exponent(emax[f]) && (m[f].m | m[f].z) != 0;
-      emax[f] += FX_HEAD;
-      ok &= emax[f] <= FX_EMAX;
+      ok &= m[f].corners(emax[f]);
       over[f] = 0;
     }
     return ok;
@@ -362,7 +360,7 @@ struct FxRawSrc4 {
     over = max(over, (uint32_t)u.x & 0x7fffffffu);
     fx_sample(fx_pair((uint32_t)u.y, (uint32_t)u.x), emax, *h, *l);
   }
-  __device__ __forceinline__ bool fit() const { return (int)((over + 1) >> 20) <= emax; }
+  __device__ __forceinline__ bool fit() const { return fx_fits(over, emax); }
   __device__ __forceinline__ bool scale() {
     FxMax m;
 #pragma unroll
@@ -370,10 +368,8 @@ struct FxRawSrc4 {
       const int2 u = v[at(1 + ((c >> 1) & 1), 1 + ((c >> 2) & 1), 1 + (c >> 3)) + 1 + (c & 1)];
       m.add((uint32_t)u.x, (uint32_t)u.y);
     }
-    bool ok = m.exponent(emax) && (m.m | m.z) != 0;
-    emax += FX_HEAD;
     over = 0;
-    return ok && emax <= FX_EMAX;
+    return m.corners(emax);
   }
 };
 
