@@ -535,6 +535,7 @@ template <int N>
 struct EvalArgs {
   int64_t c[N];
   double frac[N], inv_h[N];
+  bool finite;  // the block is known to be finite (part of a staged tile in the scaling)
 };
 template <int F, int N>
 struct EvalOut {
@@ -620,8 +621,9 @@ static __device__ __noinline__ EvalOut<F, 3> eval_otf3_full(const double *grid, 
   src.p = grid + ((in.c[2] * ny + in.c[1]) * nx + in.c[0]) * STEP;
   src.sy = nx * STEP;
   src.sz = nx * ny * STEP;
-  if (!src.template scale<true>()) return eval_otf3_f64<F, STEP>(grid, nx, ny, in);
-  if (at_node<3>(in.frac)) {
+  const bool node = at_node<3>(in.frac);
+  if (!(node && in.finite) && !src.template scale<true>()) return eval_otf3_f64<F, STEP>(grid, nx, ny, in);
+  if (node) {
     const double *p = src.at(1, 1, 1);
     EvalOut<F, 3> o;
 #pragma unroll
@@ -645,8 +647,10 @@ static __device__ __noinline__ EvalOut<F, 3> eval_otf3_full(const double *grid, 
 
 template <int F, int STEP = F>
 __device__ __forceinline__ void eval_otf3_slow(const arb_grid &g, const KParams &kp, const int64_t c[3],
-                                               const double frac[3], double val[F], double grad[3]) {
+                                               const double frac[3], double val[F], double grad[3],
+                                               bool finite = false) {
   EvalArgs<3> in;
+  in.finite = finite;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     in.c[a] = c[a];
@@ -1065,8 +1069,9 @@ template <bool GRADF>
 static __device__ __noinline__ EvalOut<1, 4> eval_otf4_full(Grid4Ref r, EvalArgs<4> in) {
   FxGrid4 src;
   r.block(src, in.c);
-  if (!src.scale<true>()) return eval_otf4_f64(r.grid, r.nx, r.ny, r.nz, r.F, r.f, GRADF, in);
-  if (at_node<4>(in.frac)) {
+  const bool node = at_node<4>(in.frac);
+  if (!(node && in.finite) && !src.scale<true>()) return eval_otf4_f64(r.grid, r.nx, r.ny, r.nz, r.F, r.f, GRADF, in);
+  if (node) {
     const double *p = src.at(1, 1, 1, 1);
     EvalOut<1, 4> o;
     o.val[0] = __ldg(p);
@@ -1089,8 +1094,10 @@ static __device__ __noinline__ EvalOut<1, 4> eval_otf4_full(Grid4Ref r, EvalArgs
 
 template <bool GRADF>
 __device__ __forceinline__ void eval_otf4_slow(const arb_grid &g, const KParams &kp, int F, int f, const int64_t c[4],
-                                               const double frac[4], double &val, double grad[4]) {
+                                               const double frac[4], double &val, double grad[4],
+                                               bool finite = false) {
   EvalArgs<4> in;
+  in.finite = finite;
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     in.c[a] = c[a];

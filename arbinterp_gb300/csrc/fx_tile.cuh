@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
           }
         }
       }
-      if (!fine) eval_otf3_slow<F>(g, kp, c, fr, val, grad);
+      if (!fine) eval_otf3_slow<F>(g, kp, c, fr, val, grad, ok);
       write_vals<3, F>(o, q.row, val, grad);
     }
   }
@@ -501,14 +501,14 @@ __global__ void __launch_bounds__(FX_THREADS, 2) eval_fx4_kernel(arb_grid g, KPa
 #pragma unroll 1
       for (int f = 0; f < NV; ++f) {
         double v = 0.0, none[4];
-        if (!contract(std::false_type(), f, v, none)) eval_otf4_slow<false>(g, kp, F, f, c, fr, v, none);
+        if (!contract(std::false_type(), f, v, none)) eval_otf4_slow<false>(g, kp, F, f, c, fr, v, none, ok);
 #pragma unroll
         for (int m = 0; m < NV; ++m)
           if (m == f) val[m] = v;
       }
       if constexpr (F != 3) {
         if (!contract(std::true_type(), F - 1, val[F - 1], grad))
-          eval_otf4_slow<true>(g, kp, F, F - 1, c, fr, val[F - 1], grad);
+          eval_otf4_slow<true>(g, kp, F, F - 1, c, fr, val[F - 1], grad, ok);
       }
       write_vals<4, F>(o, q.row, val, grad);
     }
