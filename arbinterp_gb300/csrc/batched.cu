@@ -16,7 +16,10 @@
 
 namespace arb {
 
-// Axis a of the kernel parameters of grid g (make_kparams, on the device).
+// Axis a of the kernel parameters of grid g (make_kparams, on the device); the
+// float64 step's constants (128-bit corrections of a reciprocal) only where a
+// float64 query reads them: on every tile of a mixed batch they cost 3-5 %.
+template <bool MIXED>
 __device__ void make_kparams_axis(const arb_grid &g, int a, KParams &kp) {
   const double h = a < g.dim ? g.h[a] : 1.0;
   const double lo = a < g.dim ? g.lo[a] : 0.0, hi = a < g.dim ? g.hi[a] : 0.0;
@@ -27,7 +30,7 @@ __device__ void make_kparams_axis(const arb_grid &g, int a, KParams &kp) {
   kp.ax[a].h = h;
   kp.ax[a].inv_h = 1.0 / h;
   fast_axis_pairs(kp.ax[a], lo, hi, h);
-  fast_axis_fx(kp.ax[a], h);
+  if constexpr (!MIXED) fast_axis_fx(kp.ax[a], h);
 }
 
 // One warp takes the next tile from the counter and fills descriptor slot
@@ -42,6 +45,7 @@ struct TileSlot {
   int32_t field;
 };
 
+template <bool MIXED>
 __device__ __forceinline__ void acquire_tile(const arb_grid *grids, int32_t nfields, const int64_t *tile_off,
                                              int64_t ntiles, unsigned long long *counter, TileSlot &ts) {
   const int lane = threadIdx.x & 31;
@@ -65,7 +69,7 @@ __device__ __forceinline__ void acquire_tile(const arb_grid *grids, int32_t nfie
     const uint64_t *w = reinterpret_cast<const uint64_t *>(&src);
     uint64_t *d = reinterpret_cast<uint64_t *>(&ts.g);
     for (int k = lane; k < (int)(sizeof(arb_grid) / 8); k += 32) d[k] = w[k];
-    if (lane < 4) make_kparams_axis(src, lane, ts.kp);
+    if (lane < 4) make_kparams_axis<MIXED>(src, lane, ts.kp);
     if (lane == 0) ts.field = lo;
   }
   if (lane == 0) ts.tile = tile;
@@ -106,13 +110,13 @@ __global__ void __launch_bounds__(256, 2) batched_kernel(const arb_grid *grids, 
                                                       int64_t qs, int wb, arb_query_out o,
                                                       unsigned long long *counter, int32_t *status) {
   __shared__ TileSlot slots[2];
-  if (threadIdx.x < 32) acquire_tile(grids, nfields, tile_off, ntiles, counter, slots[0]);
+  if (threadIdx.x < 32) acquire_tile<MIXED>(grids, nfields, tile_off, ntiles, counter, slots[0]);
   __syncthreads();
   for (int cur = 0;; cur ^= 1) {
     const TileSlot &ts = slots[cur];
     const int64_t tile = ts.tile;
     if (tile >= ntiles) break;
-    if (threadIdx.x < 32) acquire_tile(grids, nfields, tile_off, ntiles, counter, slots[cur ^ 1]);
+    if (threadIdx.x < 32) acquire_tile<MIXED>(grids, nfields, tile_off, ntiles, counter, slots[cur ^ 1]);
     const int32_t f = ts.field;
     const int64_t q0 = q_off[f] + (tile - tile_off[f]) * tile_rows;
     const int64_t q1 = min(q0 + (int64_t)tile_rows, q_off[f + 1]);
