@@ -535,7 +535,6 @@ template <int N>
 struct EvalArgs {
   int64_t c[N];
   double frac[N], inv_h[N];
-  bool finite;  // the block is known to be finite (part of a staged tile in the scaling)
 };
 template <int F, int N>
 struct EvalOut {
@@ -611,6 +610,25 @@ __device__ __forceinline__ bool at_node(const double frac[N]) {
 __device__ __forceinline__ double node_slope(const double *p, int64_t step, double inv_h) {
   return (0.5 * __ldg(p + step) - 0.5 * __ldg(p - step)) * inv_h;
 }
+// p: the point's F fields; steps to its neighbours in doubles.
+template <int F>
+__device__ __forceinline__ void eval_node3(const double *p, int64_t sx, int64_t sy, int64_t sz, const double *inv_h,
+                                           double val[F], double grad[3]) {
+#pragma unroll
+  for (int f = 0; f < F; ++f) val[f] = __ldg(p + f);
+  if (F != 3) {
+    grad[0] = node_slope(p + F - 1, sx, inv_h[0]);
+    grad[1] = node_slope(p + F - 1, sy, inv_h[1]);
+    grad[2] = node_slope(p + F - 1, sz, inv_h[2]);
+  }
+}
+// The corner of cell c.
+template <int F>
+__device__ __forceinline__ void eval_node3(const arb_grid &g, const int64_t c[3], const double *inv_h, double val[F],
+                                           double grad[3]) {
+  const int64_t sy = g.n[0] * F, sz = g.n[1] * sy;
+  eval_node3<F>(g.grid64 + (c[2] + 1) * sz + (c[1] + 1) * sy + (c[0] + 1) * F, F, sy, sz, inv_h, val, grad);
+}
 
 // The block as a whole sets the scale: blocks with a sample far above the
 // query's own cell; or float64 arithmetic where the scaling does not hold; or a
@@ -621,16 +639,11 @@ static __device__ __noinline__ EvalOut<F, 3> eval_otf3_full(const double *grid, 
   src.p = grid + ((in.c[2] * ny + in.c[1]) * nx + in.c[0]) * STEP;
   src.sy = nx * STEP;
   src.sz = nx * ny * STEP;
-  const bool node = at_node<3>(in.frac);
-  if (!(node && in.finite) && !src.template scale<true>()) return eval_otf3_f64<F, STEP>(grid, nx, ny, in);
-  if (node) {
-    const double *p = src.at(1, 1, 1);
+  if (!src.template scale<true>()) return eval_otf3_f64<F, STEP>(grid, nx, ny, in);
+  if (at_node<3>(in.frac)) {
     EvalOut<F, 3> o;
-#pragma unroll
-    for (int f = 0; f < F; ++f) o.val[f] = __ldg(p + f);
-    o.grad[0] = node_slope(p + F - 1, STEP, in.inv_h[0]);
-    o.grad[1] = node_slope(p + F - 1, src.sy, in.inv_h[1]);
-    o.grad[2] = node_slope(p + F - 1, src.sz, in.inv_h[2]);
+    o.grad[0] = o.grad[1] = o.grad[2] = 0.0;
+    eval_node3<F>(src.at(1, 1, 1), STEP, src.sy, src.sz, in.inv_h, o.val, o.grad);
     return o;
   }
   FxW wx, wy, wz;
@@ -647,10 +660,8 @@ static __device__ __noinline__ EvalOut<F, 3> eval_otf3_full(const double *grid, 
 
 template <int F, int STEP = F>
 __device__ __forceinline__ void eval_otf3_slow(const arb_grid &g, const KParams &kp, const int64_t c[3],
-                                               const double frac[3], double val[F], double grad[3],
-                                               bool finite = false) {
+                                               const double frac[3], double val[F], double grad[3]) {
   EvalArgs<3> in;
-  in.finite = finite;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     in.c[a] = c[a];
@@ -1056,6 +1067,7 @@ struct Grid4Ref {
   const double *grid;
   int64_t nx, ny, nz;
   int F, f;
+  bool finite;  // the block is known to be finite (part of a staged tile in the scaling)
   __device__ __forceinline__ void block(FxGrid4 &src, const int64_t c[4]) const {
     src.p = grid + (((c[3] * nz + c[2]) * ny + c[1]) * nx + c[0]) * F + f;
     src.step = F;
@@ -1070,7 +1082,7 @@ static __device__ __noinline__ EvalOut<1, 4> eval_otf4_full(Grid4Ref r, EvalArgs
   FxGrid4 src;
   r.block(src, in.c);
   const bool node = at_node<4>(in.frac);
-  if (!(node && in.finite) && !src.scale<true>()) return eval_otf4_f64(r.grid, r.nx, r.ny, r.nz, r.F, r.f, GRADF, in);
+  if (!(node && r.finite) && !src.scale<true>()) return eval_otf4_f64(r.grid, r.nx, r.ny, r.nz, r.F, r.f, GRADF, in);
   if (node) {
     const double *p = src.at(1, 1, 1, 1);
     EvalOut<1, 4> o;
@@ -1097,14 +1109,13 @@ __device__ __forceinline__ void eval_otf4_slow(const arb_grid &g, const KParams 
                                                const double frac[4], double &val, double grad[4],
                                                bool finite = false) {
   EvalArgs<4> in;
-  in.finite = finite;
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     in.c[a] = c[a];
     in.frac[a] = frac[a];
     in.inv_h[a] = kp.inv_h[a];
   }
-  const EvalOut<1, 4> o = eval_otf4_full<GRADF>(Grid4Ref{g.grid64, g.n[0], g.n[1], g.n[2], F, f}, in);
+  const EvalOut<1, 4> o = eval_otf4_full<GRADF>(Grid4Ref{g.grid64, g.n[0], g.n[1], g.n[2], F, f, finite}, in);
   val = o.val[0];
   if (GRADF) {
 #pragma unroll
@@ -1117,7 +1128,7 @@ template <bool GRADF>
 __device__ __forceinline__ void eval_otf4_fx(const arb_grid &g, const KParams &kp, int F, int f, const int64_t c[4],
                                              const FxW w[2], const double frac[4], double &val, double grad[4]) {
   FxGrid4 src;
-  Grid4Ref{g.grid64, g.n[0], g.n[1], g.n[2], F, f}.block(src, c);
+  Grid4Ref{g.grid64, g.n[0], g.n[1], g.n[2], F, f, false}.block(src, c);
   bool ok = !at_node<4>(frac) && src.scale<false>();
   if (ok) {
     long long R, G[4];

@@ -314,7 +314,12 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
           }
         }
       }
-      if (!fine) eval_otf3_slow<F>(g, kp, c, fr, val, grad, ok);
+      if (!fine) {
+        if (ok && at_node<3>(fr))  // the tile is finite: no scan of the block
+          eval_node3<F>(g, c, kp.inv_h, val, grad);
+        else
+          eval_otf3_slow<F>(g, kp, c, fr, val, grad);
+      }
       write_vals<3, F>(o, q.row, val, grad);
     }
   }
