@@ -186,13 +186,12 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
   const QRec64<3> *recs = reinterpret_cast<const QRec64<3> *>(w.rec);
   const int64_t nx = g.n[0], ny = g.n[1], nz = g.n[2];
   const BinItems items(w, bg, share);
-  for (int64_t it = blockIdx.x; it < items.n; it += gridDim.x) {
+  for (uint32_t it = blockIdx.x; it < items.n; it += gridDim.x) {
     uint32_t t0, t1;
-    const int64_t b = items.get(it, t0, t1);
+    const uint32_t b = (uint32_t)items.get(it, t0, t1), nb0 = (uint32_t)bg.nb[0], nb1 = (uint32_t)bg.nb[1],
+                   r = b / nb0;
     if (t0 == t1) continue;
-    const int64_t r = b / bg.nb[0];
-    const int og[3] = {(int)((b % bg.nb[0]) * BIN_EDGE), (int)((r % bg.nb[1]) * BIN_EDGE),
-                       (int)((r / bg.nb[1]) * BIN_EDGE)};
+    const int og[3] = {(int)((b % nb0) * BIN_EDGE), (int)((r % nb1) * BIN_EDGE), (int)((r / nb1) * BIN_EDGE)};
     if (threadIdx.x < F) smax.m[threadIdx.x] = smax.z[threadIdx.x] = 0;
     // the footprint in registers (all loads in flight at once), its largest
     // samples, then its words in shared memory

@@ -529,14 +529,14 @@ __global__ void __launch_bounds__(256) split_kernel(const uint32_t *offs, BinGeo
 struct BinItems {
   const uint32_t *offs;
   const uint2 *more;
-  int64_t nmore, n;
+  uint32_t nmore, n;  // (a grid has fewer than 2^28 bins of the staged shape)
   uint32_t share;
   int cls;
   __device__ __forceinline__ BinItems(const SortedWork &w, const BinGeom &bg, uint32_t share_)
       : offs(w.offs), more(reinterpret_cast<const uint2 *>(w.hist + 2)), share(share_), cls(bg.cls) {
     const uint32_t head = w.hist[0];
     nmore = head & ~CLASSED;
-    n = head & CLASSED ? nmore + bg.nbins : 0;
+    n = head & CLASSED ? nmore + (uint32_t)bg.nbins : 0;
   }
   // First record that needs no evaluation (of nq).
   __device__ __forceinline__ int64_t special(const BinGeom &bg, int64_t nq) const {
@@ -546,7 +546,7 @@ struct BinItems {
   __device__ __forceinline__ int64_t get(int64_t i, uint32_t &t0, uint32_t &t1) const {
     t0 = t1 = 0;
     if (i >= n) return 0;
-    int64_t b = i - nmore;
+    int64_t b = i - (int64_t)nmore;
     uint32_t part = 0;
     if (b < 0) {
       const uint2 m = more[i];
