@@ -101,7 +101,7 @@ class BatchedTricubic:
 
     def tune(self, q, counts, expected_reuse=1):
         """Pick the tile size and table threshold for this batch by timing."""
-        key = (f"batched|{torch.cuda.get_device_name(self.device)}|{self.precision}|F{self.F}|"
+        key = (f"batched|{torch.cuda.get_device_name(self.device)}|k{autotune.KERNELS}|{self.precision}|F{self.F}|"
                f"n{len(self.interps)}|rows2^{int(np.log2(max(int(np.sum(counts)), 1)))}|reuse{expected_reuse}")
         cached = autotune._MEM.get(key) or autotune._load().get(key)
         if cached:
