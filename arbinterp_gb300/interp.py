@@ -842,8 +842,10 @@ class _Interpolant:
         nsteps steps of dt, and with record_every > 0 also the path
         (nsteps // record_every, N, 6) of (x, v) states; arrays of the input
         kind.  Particles that leave the interpolation volume come back NaN;
-        `self.lost` counts them.  spatial_sort: integrate in Z-order (the
-        results are returned in the caller's order either way)."""
+        `self.lost` counts them.  spatial_sort: neighbouring threads take
+        neighbouring particles, in Z-order or, from 131,072 particles up, by
+        x-rows of cells inside 16-cell cubes (the results are returned in the
+        caller's order either way)."""
         if self._dim != 3:
             raise NotImplementedError("trajectories are built for 3D fields")
         if self._kind == _lib.KIND_VECTOR:
@@ -871,8 +873,12 @@ class _Interpolant:
         # |B| as (hi, lo) pairs costs one pass over the grid (28 bytes a point,
         # ~6 ps) and saves ~40 ps a field evaluation
         if prec == _lib.PREC_MIXED and self._F == 4 and 8 * n * int(nsteps) >= self._npts:
-            pairs = torch.empty(2 * self._npts, dtype=torch.float32, device=dev)
-            check(L.arb_norm_pairs(self._g, pairs.data_ptr(), _stream()), "arb_norm_pairs")
+            try:
+                pairs = torch.empty(2 * self._npts, dtype=torch.float32, device=dev)
+            except torch.OutOfMemoryError:
+                pass            # a grid that leaves no room for them: read from its rows, the same results
+            else:
+                check(L.arb_norm_pairs(self._g, pairs.data_ptr(), _stream()), "arb_norm_pairs")
         check(L.arb_rk4_trajectories_ordered(self._g, prec, _ptr(pairs), _ptr(order), state.data_ptr(), n, float(dt),
                                              int(nsteps), float(coef), grav, _ptr(path),
                                              int(record_every) if nrec else 0, lost.data_ptr(), _stream()),
