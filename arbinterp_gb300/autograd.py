@@ -72,11 +72,15 @@ class TricubicFunction(torch.autograd.Function):
                 None if qg is None else qg.data_ptr())
         binned = ctx.field.binned_adjoint
         if binned is None:
-            # grouping costs the binning passes, each bin's tile and one flush
-            # of its 1331 points: it pays from a sixth of the cells (86 queries
-            # a bin) on large sets (128^3: 5e5 queries 136 against 185 us, 2.5e5
-            # 108 against 99), on smaller ones from one query per cell
-            binned = n >= max(interp.sort_threshold, min(interp.nc, max(interp.nc // 6, 1 << 17)))
+            # grouping costs the binning passes (seven launches), each bin's
+            # tile and one flush of its 1331 points: it pays from a sixth of
+            # the cells (86 queries a bin), or from one query per cell on
+            # small grids, and not below 2^18 rows between the two.  Backward
+            # on the device, plain : grouped, uniform queries and a cloud of
+            # an eighth of the box: 96^3 1.35e5 rows 70 : 83 and 84 : 106 us,
+            # 2e5 95 : 93 and 110 : 120, 2.7e5 121 : 105 and 151 : 134;
+            # 128^3 2.7e5 121 : 121 and 129 : 141, 4e5 164 : 137 and 180 : 165
+            binned = n >= max(interp.sort_threshold, min(interp.nc, max(interp.nc // 6, 1 << 18)))
         if mixed and binned:
             # grouped by bin: dL/df accumulated per bin in shared memory
             need = int(L.arb_adjoint_work_bytes(interp._g, n))
