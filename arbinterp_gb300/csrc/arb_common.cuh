@@ -120,8 +120,8 @@ struct FastAxis {
   double lo, h, inv_h;
   float loh, lol, ih, il;             // float32 pairs of IntMin and 1/h
   int df;                             // the float32 double-float step applies on this axis
-  unsigned long long hm, hinv;        // significand of h (53 bits) and floor(2^115 / hm), for axis_step_fx
-  int he;                             // biased exponent of h; 0 where axis_step_fx does not apply
+  unsigned long long hm, hinv;        // significand of h (53 bits) and floor(2^115 / hm), for fx_quotient
+  int he;                             // biased exponent of h; 0 where fx_quotient does not apply
 };
 
 // Range of the axis as keys, finite so that every NaN lies outside.  The keys tell
@@ -134,7 +134,7 @@ __host__ __device__ __forceinline__ void fast_axis_range(FastAxis &f, unsigned l
   f.hi_key = ord_key_bits(hi) < pinf ? ord_key_bits(hi) : pinf;
 }
 
-// Constants of axis_step_fx: h normal, finite and positive.  floor(2^115 / hm)
+// Constants of fx_quotient: h normal, finite and positive.  floor(2^115 / hm)
 // by a float64 quotient (53 of its 63 bits) and two integer corrections.
 __host__ __device__ inline void fast_axis_fx(FastAxis &f, double h) {
 #ifdef __CUDA_ARCH__

@@ -34,7 +34,11 @@ __global__ void __launch_bounds__(256) norm_pairs_kernel(const float *g32, int64
 // just past a row of cubes has a few warps with one cell of every row, though,
 // and where an SM holds few warps the slowest one counts: 2e4 x 20 on 64^3 467 : 427
 // or 449 : 559 us, 4e4 516 : 646.  So Z-order over the box (10 bits an axis)
-// below CELLS_FROM particles.
+// below CELLS_FROM particles: 77,824 are the 16 warps of every SM, and from 1.4e5 the
+// x-rows win at most densities (10 steps, uniform in 0.6 of the box: 64^3 628 : 575,
+// 128^3 673 : 590, 256^3 1313 : 1273; 1e6 2419 : 2316, 3025 : 2321, 3185 : 2588; a tight
+// cloud 64^3 562 : 554, 128^3 652 : 588, 256^3 1022 : 917) and lose at most 6 % in
+// the densest (1e6 in a cloud of 16 cells' width on 64^3: 2206 : 2341).
 constexpr int64_t CELLS_FROM = 1 << 17;
 __device__ __forceinline__ uint32_t spread10(uint32_t v) {
   v = (v | v << 16) & 0x030000ffu;

@@ -51,8 +51,8 @@ struct __align__(DIM == 3 ? 32 : 8) QRec64 {
 };
 static_assert(sizeof(QRec) == 32 && sizeof(QRec64<3>) == 32 && sizeof(QRec64<4>) == 40, "record sizes");
 
-// Index of a float64 record that needs no evaluation: NaN_CELL (out of volume
-// or a NaN row), NaN_CELL - 1 (the reference's sentinel column).
+// Index of a float64 record that needs no evaluation: NAN_CELL (out of volume
+// or a NaN row), NAN_CELL - 1 (the reference's sentinel column).
 template <int DIM>
 constexpr unsigned long long NAN_CELL = (1ULL << (32 + 2 * DIM)) - 1ULL;
 
