@@ -424,7 +424,8 @@ __device__ __forceinline__ bool axis_step_df(float qh, float ql, const FastAxis 
   const float ph = __fmul_rn(sh, ax.ih);
   const float pe = __fmaf_rn(sh, ax.ih, -ph);
   const float pl = __fmaf_rn(sh, ax.il, __fmaf_rn(st, ax.ih, pe));
-  float kf = __fsub_rn(__fadd_rd(ph, 8388608.f), 8388608.f);  // floor (0 <= ph < 2^21)
+  // floor for 0 <= ph < 2^21; a ph that rounded below 0 gives -0.5, so false below
+  float kf = __fsub_rn(__fadd_rd(ph, 8388608.f), 8388608.f);
   fr = __fadd_rn(__fsub_rn(ph, kf), pl);
   const float up = fr < 0.f ? -1.f : fr >= 1.f ? 1.f : 0.f;
   kf = __fadd_rn(kf, up);

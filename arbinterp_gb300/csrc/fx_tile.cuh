@@ -16,7 +16,8 @@
 // (steep fields far from their peak) the tile keeps the float64 samples and
 // every query sets the scale from its own cell's corners, converting as it
 // reads.  A query that this does not hold either (FX_HEAD), and bins with
-// samples outside the scaling, go to eval_otf3_slow / eval_otf4_slow.
+// samples outside the scaling, go to eval_otf3_slow / eval_otf4_slow; a query on a
+// grid point takes its samples as they are (eval_node3, eval_otf4_slow).
 #pragma once
 
 namespace arb {
