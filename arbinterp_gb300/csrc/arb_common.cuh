@@ -326,25 +326,11 @@ __device__ __forceinline__ int64_t flat_step(const int32_t fl[4], const arb_grid
   return (int64_t)idx;
 }
 
-// Floors that 32 bits do not hold (an axis whose first spacing is tiny): the
-// floor saturates, past every cell of its axis, and the index is formed from the
-// 64-bit floors, saturated far past every table.
+// Floors that 32 bits do not hold (an axis whose first spacing is tiny) saturate:
+// past every cell of their axis.  The rows' indices are then beyond the table by
+// themselves below 2^31 - 1 cells, and set so on larger grids.
 __device__ __forceinline__ int32_t narrow_floor(int64_t k) {
   return (unsigned long long)k > 0x7fffffffULL ? 0x7fffffff : (int32_t)k;
-}
-template <int DIM>
-struct WideSteps {
-  int64_t k[DIM], m[DIM];  // floors, cells per axis
-};
-template <int DIM>
-static __device__ __noinline__ int64_t wide_index(WideSteps<DIM> w) {
-  unsigned long long idx = 0;
-#pragma unroll 1
-  for (int a = DIM - 1; a >= 0; --a) {
-    const unsigned __int128 v = (unsigned __int128)idx * (unsigned long long)w.m[a] + (unsigned long long)w.k[a];
-    idx = v > (1ULL << 62) ? 1ULL << 62 : (unsigned long long)v;
-  }
-  return (int64_t)idx;
 }
 
 struct AxisStep64 {
@@ -386,27 +372,19 @@ __device__ __forceinline__ CoordStep coord_step_fx(const double *qrow, const Fas
     s.idx = g.nc;
     return s;
   }
+  bool wide = false;
   if (slow) {
-    WideSteps<DIM> w;
-    bool wide = false;
 #pragma unroll
-    for (int a = 0; a < DIM; ++a) {
-      w.k[a] = s.fl[a];
-      w.m[a] = g.n[a] - 3;
+    for (int a = 0; a < DIM; ++a)
       if (!fine[a]) {
         const AxisStep64 r = axis_step_div(__dsub_rn(qrow[a], ax[a].lo), ax[a].h);
-        w.k[a] = (int64_t)r.k;
-        s.fl[a] = narrow_floor(w.k[a]);
+        s.fl[a] = narrow_floor((int64_t)r.k);
         frac[a] = r.frac;
+        wide |= s.fl[a] == 0x7fffffff;
       }
-      wide |= s.fl[a] != w.k[a];
-    }
-    if (wide) {
-      s.idx = wide_index<DIM>(w);
-      return s;
-    }
   }
   s.idx = flat_step<DIM>(s.fl, g);
+  if (wide && s.idx <= g.nc) s.idx = g.nc + 1;
   return s;
 }
 
@@ -479,27 +457,19 @@ __device__ __forceinline__ CoordStep coord_step_fast(const double *qrow, const F
     s.idx = g.nc;
     return s;
   }
+  bool wide = false;
   if (slow) {
-    WideSteps<DIM> w;
-    bool wide = false;
 #pragma unroll
-    for (int a = 0; a < DIM; ++a) {
-      w.k[a] = s.fl[a];
-      w.m[a] = g.n[a] - 3;
+    for (int a = 0; a < DIM; ++a)
       if (!fine[a]) {
         const AxisStep r = axis_step_rest(qrow[a], ax[a]);
-        w.k[a] = r.k;
-        s.fl[a] = narrow_floor(w.k[a]);
+        s.fl[a] = narrow_floor(r.k);
         frac[a] = r.fr;
+        wide |= s.fl[a] == 0x7fffffff;
       }
-      wide |= s.fl[a] != w.k[a];
-    }
-    if (wide) {
-      s.idx = wide_index<DIM>(w);
-      return s;
-    }
   }
   s.idx = flat_step<DIM>(s.fl, g);
+  if (wide && s.idx <= g.nc) s.idx = g.nc + 1;
   return s;
 }
 
