@@ -273,10 +273,11 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
     __syncthreads();
     // the next record is loaded while this one is evaluated
     QRec64<3> next;
-    if (threadIdx.x < t1 - t0) next = recs[t0 + threadIdx.x];
-    for (uint32_t t = t0 + threadIdx.x; t - t0 < t1 - t0; t += FX_THREADS) {
+    const uint32_t first = t0 + threadIdx.x;
+    if (first < t1) next = recs[first];
+    for (uint32_t t = first; t < t1; t += FX_THREADS) {
       const QRec64<3> q = next;
-      if (t + FX_THREADS - t0 < t1 - t0) next = recs[t + FX_THREADS];
+      if (t + FX_THREADS < t1) next = recs[t + FX_THREADS];
       int64_t c[3];
       cell_coords<3>((int64_t)rec64_cell<3>(q), g, c);
       const double fr[3] = {rec64_frac<3>(q, 0), rec64_frac<3>(q, 1), rec64_frac<3>(q, 2)};
@@ -461,7 +462,8 @@ __global__ void __launch_bounds__(FX_THREADS, 2) eval_fx4_kernel(arb_grid g, KPa
         }
     }
     __syncthreads();
-    for (uint32_t t = t0 + threadIdx.x; t - t0 < t1 - t0; t += FX_THREADS) {
+    const uint32_t first = t0 + threadIdx.x;
+    for (uint32_t t = first; t < t1; t += FX_THREADS) {
       const QRec64<4> q = recs[t];
       int64_t c[4];
       cell_coords<4>((int64_t)rec64_cell<4>(q), g, c);

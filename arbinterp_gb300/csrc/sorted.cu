@@ -789,10 +789,10 @@ __global__ void __launch_bounds__(BINC_THREADS, F == 4 ? 3 : (F == 3 ? 5 : 4)) e
     if (t1 > t0) {
       // the next record is loaded while this one is evaluated
       QRec rnext;
-      if (threadIdx.x < t1 - t0) rnext = recs[t0 + threadIdx.x];
-      for (uint32_t t = t0 + threadIdx.x; t - t0 < t1 - t0; t += BINC_THREADS) {
+      if (t0 + threadIdx.x < t1) rnext = recs[t0 + threadIdx.x];
+      for (uint32_t t = t0 + threadIdx.x; t < t1; t += BINC_THREADS) {
         const QRec r = rnext;
-        if (t + BINC_THREADS - t0 < t1 - t0) rnext = recs[t + BINC_THREADS];
+        if (t + BINC_THREADS < t1) rnext = recs[t + BINC_THREADS];
         int64_t c[3];
         unpack_cell<3>(r.cell, c);
         const int bi = (((int)c[2] - og[2]) * TILE_EDGE + ((int)c[1] - og[1])) * TILE_EDGE + ((int)c[0] - og[0]);
@@ -971,7 +971,7 @@ __global__ void __launch_bounds__(BIN4_THREADS, 4) eval_bin4_kernel(arb_grid g, 
     if (t1 > t0) {
       int64_t og[4];
       bin_origin4(b, bg, og);
-      for (uint32_t t = t0 + threadIdx.x; t - t0 < t1 - t0; t += BIN4_THREADS) {
+      for (uint32_t t = t0 + threadIdx.x; t < t1; t += BIN4_THREADS) {
         const QRec r = recs[t];
         int64_t c[4];
         unpack_cell<4>(r.cell, c);
@@ -1155,7 +1155,7 @@ static void launch_eval(const arb_grid *g, const KParams &kp, int64_t nq, const 
   const BinGeom bg = bin_geom(g, MIXED ? ARB_PREC_MIXED : ARB_PREC_FP64, nq);
   const int TE = DIM == 3 ? 256 : 128;
   bool staged = false;
-  if (!table) {
+  if (!table && nq <= STAGED_ROWS) {
     if constexpr (!MIXED)
       staged = launch_eval_fx<DIM>(g, kp, bg, nq, out, w, s);
     else if constexpr (DIM == 3)

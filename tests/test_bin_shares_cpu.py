@@ -16,7 +16,7 @@ using namespace arb;
 
 int main() {
   const int64_t top = 0xffffffffLL;
-  const int64_t counts[] = {1, 511, 512, 513, 4097, 1000003, 3000000000LL, top - 700, top - 1, top};
+  const int64_t counts[] = {1, 511, 512, 513, 4097, 1000003, 3000000000LL, top - 1025, STAGED_ROWS, top - 1, top};
   const int64_t bins[] = {1, 2, 7, 600, 1215, 1216, 32768, 1000000};
   for (int64_t nq : counts)
     for (int64_t nb : bins) {
@@ -37,9 +37,10 @@ int main() {
                           (long long)n, (long long)end, (long long)p, t0, t1);
               return 2;
             }
-            int64_t steps = 0;  // of the last of 256 threads, as the kernels count
+            int64_t steps = 0;  // of the last of 256 threads, as the adjoint counts
             for (uint32_t t = t0 + 255; t - t0 < t1 - t0; t += 256) ++steps;
             if (steps != (int64_t)(t1 - t0) / 256) return 5;
+            if (nq <= STAGED_ROWS && t1 > 0xffffffffu - 512) return 6;  // and the evaluators: no record past the end wraps
             at = t1;
           }
           if (at != end) return 3;
