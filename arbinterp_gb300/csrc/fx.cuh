@@ -179,7 +179,7 @@ __host__ __device__ __forceinline__ void fx_axis(unsigned long long tbits, FxW &
 }
 
 #ifdef __CUDACC__
-// Weights of outer axes (4D: z and t; z of the 3D 'both' tiles) in shared memory, a
+// Weights of outer axes (4D: z and t; z of the 3D tiles with a gradient) in shared memory, a
 // column a thread: in registers they were 32 of the ~190 that fx_eval4 has alive, and the
 // loops over k and t picked from them by selects (1.5e6 scalar queries on 33 x 41
 // x 29 x 17, one lane a query: 1122 -> 1049 us).  Kernels that use them have at

@@ -290,12 +290,14 @@ __global__ void __launch_bounds__(FX_THREADS, F == 4 ? 3 : 4) eval_fx3_kernel(ar
         fx_axis<1>(fx_bits(fr[1]), wy);
         fx_axis<1>(fx_bits(fr[2]), wz);
         auto eval = [&](const auto &src, long long R[F], long long G[3]) {
-          if constexpr (F == 4)  // z weights from shared memory: 3215 -> 3097 us, with y's too 3092
+          // z weights from shared memory: 'both' 3215 -> 3097 us (with y's too 3092), scalar 1e6 on
+          // 101 x 87 x 93 154 -> 147; three components 818 -> 835, so those keep registers
+          if constexpr (F != 3)
             fx_eval3<F>(src, wx, wy, FxZ(), R, G);
           else
             fx_eval3<F>(src, wx, wy, wz, R, G);
         };
-        if constexpr (F == 4) FxZ::set(0, wz);
+        if constexpr (F != 3) FxZ::set(0, wz);
         long long R[F], G[3];
         if (!uneven) {
           FxTileSrc3<F> src;
